@@ -82,7 +82,9 @@ typedef struct {
                                  systems whose vector fits in shared memory (up to
                                  192 KB) sweep both factors in one CTA; otherwise
                                  FP32 factors take SENK_SWEEP_ROWS and FP64
-                                 factors SENK_SWEEP_COLOURS */
+                                 factors row-sorted slices, one launch per
+                                 colour (row slots where a group's block does
+                                 not fit shared memory) */
 #define SENK_SWEEP_COLOURS 1  /* row-slot layout, one launch per colour (level set),
                                  one CTA per group */
 #define SENK_SWEEP_DATAFLOW 2 /* compact chain layout, one launch per sweep: each

@@ -207,6 +207,12 @@ struct SweepFactor {
     // compact, per colour: every colour takes k_sweep_cc2 (SENK_SWEEP_WIDE), or
     // with rowlane every colour k_sweep_rl with two chains per lane
     bool force_wide = false;
+    // row-sorted slice layout, one launch per colour (k_sweep_lv): its groups
+    // and their blocks; `launches` gives the colours
+    bool slices = false;
+    int lv_rows = 0;               // rows per group
+    DevBuf<LvGroup> lgroups;
+    DevBuf<unsigned char> lblocks;
     // compact, per colour, external entries chain-major: k_sweep_rl (lanes =
     // rows of a chain) instead of k_sweep_cc
     bool rowlane = false;

@@ -10,6 +10,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "lv_layout.hpp"
 #include "wf_layout.hpp"
 
 namespace senkgpu {
@@ -1781,6 +1782,198 @@ k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (live[r]) y[row[r]] = a[r].out();
+}
+
+// t -= v[u] * yy[u] for the last n of B slots (1 <= n <= B; n the same in the
+// whole warp), in order. The entry into the chain is a jump: this chip runs an
+// FP64 instruction in about 19 cycles per SM (one unit, one warp instruction
+// at a time), and a predicated one costs the same when all of its lanes are
+// off (measured: 65 cycles a step in one warp either way), so slots without
+// an entry must not be issued.
+template <int B, typename VT, typename XT>
+__device__ __forceinline__ void sub_last(XT &t, const VT (&v)[B], const XT (&yy)[B], int n)
+{
+    static_assert(B == 3 || B == 6, "batches of three or six");
+    switch (n) {
+    case 6: if constexpr (B == 6) t -= (XT)v[B - 6] * yy[B - 6];
+    case 5: if constexpr (B == 6) t -= (XT)v[B - 5] * yy[B - 5];
+    case 4: if constexpr (B == 6) t -= (XT)v[B - 4] * yy[B - 4];
+    case 3: t -= (XT)v[B - 3] * yy[B - 3];
+    case 2: t -= (XT)v[B - 2] * yy[B - 2];
+    case 1: t -= (XT)v[B - 1] * yy[B - 1];
+    default: break;
+    }
+}
+
+// Resident CTAs per SM that k_sweep_lv is compiled for: 40 registers a thread.
+constexpr int lv_min_blocks(int threads) { return 1536 / threads; }
+
+// One colour per launch on the row-sorted slice layout (lv_layout.hpp), one
+// CTA per group of up to 512 rows: the distinct rows of earlier colours that
+// the group reads are gathered into shared memory, the external slices
+// subtract them (one warp per slice), then the in-chain entries follow step by
+// step (one warp per slice, a barrier among the warps that take part), and the
+// rows are stored in order.
+//
+// What bounds it is the dependent steps of a colour and, in the wide colours,
+// FP64 instructions (19 cycles of the SM's one FP64 unit per warp instruction)
+// and gather requests. So every FP64 instruction has nearly all of its lanes
+// in use, and the group's gathers are issued together, sorted, each row once.
+// FP64 application on the 128^3 convection-diffusion system 0.154 ms, on the
+// 160^3 variable-coefficient one 0.266 ms; row slots (k_sweep) 0.302 and 0.512,
+// row per lane (k_sweep_rl) 0.317 and 0.514. A colour of the 128^3 system takes
+// 4.4 us when narrow: 1.0 until the wait on the previous colour returns, 0.4
+// to 0.9 gathers, 0.5 to 1.0 external entries, 1.4 in-chain steps, 0.25 store.
+//
+// The block (TMA) and, with early_x, x and the gate are read before the
+// kernel waits for the previous one (early_x as in k_sweep_cc). A staging wait
+// that runs out sets *status = 2.
+template <typename VT, bool UPPER, int THREADS>
+__global__ void __launch_bounds__(THREADS, lv_min_blocks(THREADS))
+k_sweep_lv(const LvGroup *__restrict__ groups, int g0, const uint4 *__restrict__ blocks, const VT *x, VT *y,
+           const int *gate, int *status, int early_x)
+{
+    extern __shared__ __align__(128) unsigned char lvs[];
+    __shared__ __align__(8) unsigned long long bar;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
+    const LvGroup d = groups[g0 + blockIdx.x];
+    const unsigned bytes = (unsigned)d.units * 16u;
+    VT *ys = reinterpret_cast<VT *>(lvs + bytes);  // rows, external columns, zero
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, bytes);
+        bulk_g2s(lvs, blocks + d.off, bytes, &bar);
+    }
+    bool skip = false;
+    if (early_x) {
+        for (int i = tid; i < d.nrows; i += nt) ys[i] = x[d.pos0 + i];
+        skip = gated(gate);
+    } else {
+        pdl_launch_dependents();
+    }
+    __syncthreads();
+    const bool ok = mbar_wait_bounded(&bar, 0, kWaitLimit);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(status, 2);
+        if (!ok) mbar_wait_bounded(&bar, 0, kWaitLimit);
+        pdl_wait();
+        return;
+    }
+    const LvHeader *hd = reinterpret_cast<const LvHeader *>(lvs);
+    const int next = hd->next, ncol = hd->ncols, steps = hd->steps, most = hd->most;
+    const LvParts P = lv_parts(*hd, UPPER ? d.nrows * (unsigned)sizeof(VT) : 0u, sizeof(VT));
+    const uint32_t *word = reinterpret_cast<const uint32_t *>(hd + 1);
+    const uint16_t *first = reinterpret_cast<const uint16_t *>(lvs + P.first);
+    const uint16_t *rows = reinterpret_cast<const uint16_t *>(lvs + P.rows);
+    const uint2 *rec = reinterpret_cast<const uint2 *>(lvs + P.rec);
+    const int *cols = reinterpret_cast<const int *>(lvs + P.cols);
+    const VT *dv = reinterpret_cast<const VT *>(lvs + P.dinv);
+    const uint16_t *place = reinterpret_cast<const uint16_t *>(lvs + P.place);
+    const VT *vw = reinterpret_cast<const VT *>(lvs + P.val);
+    pdl_wait();  // the previous colour (or the producer of x) has finished
+    if (early_x) {
+        pdl_launch_dependents();
+    } else {
+        skip = gated(gate);
+        for (int i = tid; i < d.nrows; i += nt) ys[i] = x[d.pos0 + i];
+    }
+    if (skip) return;
+    {
+        constexpr int B = 4;
+        VT *ye = ys + d.nrows;
+        for (int i = tid; i < ncol; i += B * nt) {
+            VT g[B];
+#pragma unroll
+            for (int u = 0; u < B; u++)
+                if (i + u * nt < ncol) g[u] = y[cols[i + u * nt]];
+#pragma unroll
+            for (int u = 0; u < B; u++)
+                if (i + u * nt < ncol) ye[i + u * nt] = g[u];
+        }
+        if (tid == 0) ye[ncol] = VT(0);
+    }
+    __syncthreads();
+    for (int s = w; s < next; s += nw) {
+        constexpr int B = 6;
+        const uint32_t h = word[s];
+        const unsigned id = rows[s * 32 + lane];
+        const int wd = (int)(h & 255u), at = (int)((h & ~kLvFinal) >> 8) * 32 + lane;
+        VT t = id != kLvNone ? ys[id] : VT(0);
+        for (int k1 = (wd + B - 1) % B + 1; k1 <= wd; k1 += B) {  // entries up to k1, the first batch partial
+            VT yy[B], vv[B];
+#pragma unroll
+            for (int u = 0; u < B; u++)
+                if (k1 - B + u >= 0) {
+                    yy[u] = ys[place[at + (k1 - B + u) * 32]];
+                    vv[u] = vw[at + (k1 - B + u) * 32];
+                }
+            sub_last<B>(t, vv, yy, min(k1, B));
+        }
+        if (UPPER && (h & kLvFinal)) {
+            if (id != kLvNone) t *= dv[id];
+        }
+        if (id != kLvNone) ys[id] = t;
+    }
+    __syncthreads();
+    // in-chain entries: step by step
+    word += next;
+    auto solve = [&](uint32_t h, uint2 r) {
+        const int wd = (int)(h & 3u), at = (int)((h & ~kLvFinal) >> 8) * 32 + lane;
+        const unsigned row = r.x & 0xffffu;
+        VT v[3], yy[3];
+        yy[2] = ys[r.y >> 16];
+        v[2] = vw[at + (wd - 1) * 32];
+        if (wd > 1) {
+            yy[1] = ys[r.y & 0xffffu];
+            v[1] = vw[at + (wd - 2) * 32];
+        }
+        if (wd > 2) {
+            yy[0] = ys[r.x >> 16];
+            v[0] = vw[at];
+        }
+        VT t = ys[row];
+        const bool fin = UPPER && (h & kLvFinal);
+        VT di = VT(1);
+        if (fin && row < d.nrows) di = dv[row];
+        sub_last<3>(t, v, yy, wd);
+        if (fin) t *= di;
+        if (row < d.nrows) ys[row] = t;
+    };
+    if (most <= nw && steps <= 32) {
+        // one slice per warp and step at most: lane l holds the word and the
+        // number of the warp's slice at step l (-1: none), and a step's record
+        // is read during the step before it
+        if (w < most) {
+            int sl = -1;
+            uint32_t hw = 0u;
+            if (lane < steps && first[lane] + w < first[lane + 1]) {
+                sl = first[lane] + w;
+                hw = word[sl];
+            }
+            int s = __shfl_sync(0xffffffffu, sl, 0);
+            uint32_t h = __shfl_sync(0xffffffffu, hw, 0);
+            uint2 r = make_uint2(0u, 0u);
+            if (s >= 0) r = rec[s * 32 + lane];
+            for (int l = 0; l < steps; l++) {
+                const int s1 = __shfl_sync(0xffffffffu, sl, (l + 1) & 31);
+                const uint32_t h1 = __shfl_sync(0xffffffffu, hw, (l + 1) & 31);
+                uint2 r1 = r;
+                if (s1 >= 0) r1 = rec[s1 * 32 + lane];
+                if (s >= 0) solve(h, r);
+                s = s1;
+                h = h1;
+                r = r1;
+                if (l + 1 < steps) named_bar(1, most * 32);
+            }
+        }
+    } else {
+        for (int l = 0; l < steps; l++) {
+            for (int s = first[l] + w; s < first[l + 1]; s += nw) solve(word[s], rec[s * 32 + lane]);
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < d.nrows; i += nt) y[d.pos0 + i] = ys[i];
 }
 
 // Colours [cbeg, cend) of one sweep in one cooperative launch, on the

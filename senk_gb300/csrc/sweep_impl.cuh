@@ -3,15 +3,17 @@
 // GPU (replaces include/senk_sparse.hpp:132-315, SptrsvCsr_l/_u in their
 // sequential, AMC and ABMC forms).
 //
-// Two layouts. Both take chains (`bs` consecutive schedule positions, one ABMC
-// block, solved in order) 32 at a time from one colour, and keep each row's
+// Three layouts. All take chains (`bs` consecutive schedule positions, one ABMC
+// block, solved in order) from one colour into groups, and keep each row's
 // subtraction order (entries of other chains first, which are final before the
 // colour starts, then in-chain entries; each part in the reference's column
 // order: ascending for L, descending for U).
-//  * Compact chains (default for AMC/ABMC schedules, `k_sweep_wf`, one launch
-//    per sweep, one warp per group of 32 chains): each chain's entries are
-//    packed one after another, lane = chain, so a group pads only to its widest
-//    chain; the chains of a colour are sorted by their entry counts first.
+//  * Row-sorted slices (FP64 factors by default, lv_layout.hpp, `k_sweep_lv`,
+//    one launch per colour).
+//  * Compact chains (FP32 factors by default, wf_layout.hpp, 32 chains to a
+//    group): each chain's entries are packed one after another, so a group
+//    pads only to its widest chain; the chains of a colour are sorted by their
+//    entry counts first.
 //  * Row slots (`k_sweep`, one launch per colour; level-set schedules of the
 //    natural order, and SENK_SWEEP_COLOURS): slot k of row l of every chain of
 //    a group is one 32-wide column, rows padded to the group's widest.
@@ -20,6 +22,7 @@
 #include <memory>
 
 #include "device.hpp"
+#include "lv_build.cuh"
 
 namespace senkgpu {
 
@@ -182,6 +185,7 @@ void build_factor(SweepFactor<VT> &F, bool upper, int N, const VT *val, const in
     F.persistent = false;
     F.force_wide = false;
     F.rowlane = false;
+    F.slices = false;
     // Host vectors are released on return: finish the copies first.
     SENK_CUDA(cudaStreamSynchronize(s));
 }
@@ -223,6 +227,7 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.persistent = false;
     F.force_wide = false;
     F.rowlane = chain_major;
+    F.slices = false;
     F.ngroups = ng;
     F.slots_max = lay.slots_max;
     F.elems = (long long)lay.col.size();
@@ -296,6 +301,101 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
         F.ctrl.upload(ctrl0, 4, s);
     }
     SENK_CUDA(cudaStreamSynchronize(s));  // the layout's host arrays are released on return
+    return true;
+}
+
+// Most bytes of entries a group should have, so that four CTAs of k_sweep_lv
+// are resident per SM with its operands.
+constexpr size_t kLvWantBytes = 32 * 1024;
+
+// Row-sorted slice layout (lv_layout.hpp) for k_sweep_lv, built on the device
+// from the factor's arrays (on the host where a group is larger than the
+// device builder's tables). Returns false (and builds nothing) when a group
+// would not fit the shared memory even with the smallest groups.
+template <typename VT, bool UPPER>
+bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, const int *rptr,
+                     const std::vector<Group> &colours, int bs, const std::vector<int> &colour_of, cudaStream_t s)
+{
+    std::vector<std::pair<int, int>> cr;
+    for (const Group &g : colours) cr.push_back({g.p0, g.p1});
+    LvLayout<VT> lay;
+    lay.gr = lv_cut(lay.groups, lay.colour_groups, rptr, cr, bs, kLvWantBytes, sizeof(VT));
+    const int ng = (int)lay.groups.size();
+    std::vector<LvJob> jobs;
+    for (size_t c = 0; c < cr.size(); c++)
+        for (int g = lay.colour_groups[c]; g < lay.colour_groups[c + 1]; g++)
+            jobs.push_back({lay.groups[g].pos0, lay.groups[g].nrows, cr[c].first, cr[c].second});
+    const size_t nnz = (size_t)rptr[N];
+    DevBuf<VT> dval(std::max<size_t>(nnz, 1));
+    DevBuf<int> dcind(std::max<size_t>(nnz, 1)), drptr((size_t)N + 1);
+    DevBuf<LvJob> djobs(ng);
+    DevBuf<LvSize> dsize(ng);
+    dval.upload(val, nnz, s);
+    dcind.upload(cind, nnz, s);
+    drptr.upload(rptr, (size_t)N + 1, s);
+    djobs.upload(jobs.data(), jobs.size(), s);
+    constexpr int smem = (int)sizeof(LvBuildShared);
+    SENK_CUDA(cudaFuncSetAttribute(k_lv_build<VT, UPPER, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SENK_CUDA(cudaFuncSetAttribute(k_lv_build<VT, UPPER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_lv_build<VT, UPPER, false><<<ng, kLvMaxRows, smem, s>>>(djobs.p, dval.p, dcind.p, drptr.p, N, bs, nullptr,
+                                                              nullptr, dsize.p);
+    SENK_LAUNCH_CHECK();
+    std::vector<LvSize> size(ng);
+    SENK_CUDA(cudaMemcpyAsync(size.data(), dsize.p, sizeof(LvSize) * ng, cudaMemcpyDeviceToHost, s));
+    SENK_CUDA(cudaStreamSynchronize(s));
+    long long units = 0;
+    int bad = 0;
+    size_t worst = 0;
+    for (int g = 0; g < ng; g++) {
+        bad = std::max(bad, size[g].bad);
+        lay.groups[g].off = (int)units;
+        lay.groups[g].units = size[g].units;
+        worst = std::max(worst, (size_t)size[g].smem);
+        units += size[g].units;
+    }
+    bool on_host = false;
+    if (bad) {
+        // reports a row that does not fit the schedule (throws), or builds
+        // what the device builder's tables do not hold
+        if (!make_lv_layout(lay, UPPER, N, val, cind, rptr, cr, bs, colour_of.data(), kLvWantBytes, kMaxStagedBytes))
+            return false;
+        on_host = true;
+    } else {
+        if (worst > kMaxStagedBytes) return false;
+        SENK_REQUIRE(units < INT_MAX, "factor too large for 32-bit block offsets");
+        lay.bytes = (size_t)std::max<long long>(units, 1) * 16;
+        lay.colour_smem.assign(cr.size(), 0);
+        for (size_t c = 0; c < cr.size(); c++)
+            for (int g = lay.colour_groups[c]; g < lay.colour_groups[c + 1]; g++)
+                lay.colour_smem[c] = std::max(lay.colour_smem[c], (size_t)size[g].smem);
+    }
+    F.upper = UPPER;
+    F.mapped = false;
+    F.bs = bs;
+    F.slices = true;
+    F.lv_rows = lay.gr;
+    F.nnz = (long long)nnz;
+    F.colour_groups = lay.colour_groups;
+    F.lgroups.alloc(lay.groups.size());
+    F.lgroups.upload(lay.groups.data(), lay.groups.size(), s);
+    F.lblocks.alloc(lay.bytes);
+    if (on_host) {
+        F.lblocks.upload(lay.blocks.get(), lay.bytes, s);
+    } else {
+        k_lv_build<VT, UPPER, true><<<ng, kLvMaxRows, smem, s>>>(djobs.p, dval.p, dcind.p, drptr.p, N, bs, F.lgroups.p,
+                                                                 F.lblocks.p, dsize.p);
+        SENK_LAUNCH_CHECK();
+    }
+    F.launches.clear();
+    for (size_t c = 0; c + 1 < lay.colour_groups.size(); c++) {
+        typename SweepFactor<VT>::Launch L{};
+        L.g0 = lay.colour_groups[c];
+        L.g1 = lay.colour_groups[c + 1];
+        L.early_x = F.launches.empty() ? 0 : 1;
+        L.smem = lay.colour_smem[c];
+        if (L.g1 > L.g0) F.launches.push_back(L);
+    }
+    SENK_CUDA(cudaStreamSynchronize(s));  // the arrays used above are released on return
     return true;
 }
 
@@ -512,6 +612,48 @@ void shape_cc(SweepFactor<VT> &F)
     }
 }
 
+// Row-sorted slices, one launch per colour (k_sweep_lv), chained by
+// programmatic dependent launch.
+template <typename VT, bool UPPER>
+void launch_lv(const SweepFactor<VT> &F, int *status, const VT *x, VT *y, cudaStream_t s, const int *gate)
+{
+    for (const auto &L : F.launches) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(L.g1 - L.g0);
+        cfg.blockDim = dim3(L.wide ? F.lv_rows / 2 : F.lv_rows);
+        cfg.dynamicSmemBytes = L.smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        SENK_CUDA(cudaLaunchKernelEx(&cfg, L.wide ? k_sweep_lv<VT, UPPER, kLvMaxRows / 2> : k_sweep_lv<VT, UPPER, kLvMaxRows>,
+                                     (const LvGroup *)F.lgroups.p, L.g0, (const uint4 *)F.lblocks.p, x, y, gate,
+                                     status, L.early_x));
+    }
+}
+
+// Shared memory limits of k_sweep_lv, and which colours take half the threads
+// (two slices per warp): those with more groups than one wave of full-width
+// CTAs holds.
+template <typename VT, bool UPPER>
+void shape_lv(SweepFactor<VT> &F)
+{
+    auto full = k_sweep_lv<VT, UPPER, kLvMaxRows>, half = k_sweep_lv<VT, UPPER, kLvMaxRows / 2>;
+    size_t most = 48 * 1024;
+    for (const auto &L : F.launches) most = std::max(most, L.smem);
+    SENK_CUDA(cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    SENK_CUDA(cudaFuncSetAttribute(half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    if (F.lv_rows < 64) return;
+    for (auto &L : F.launches) {
+        int one = 0, two = 0;
+        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, full, F.lv_rows, L.smem));
+        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, half, F.lv_rows / 2, L.smem));
+        L.wide = (L.g1 - L.g0) > one * sm_count() && two > one ? 1 : 0;
+    }
+}
+
 // Shape of the cooperative launches: two staging buffers of the widest group's
 // block; as many CTAs fit at once as the occupancy allows. Every run of at
 // least two consecutive colours (in processing order) whose groups fit that
@@ -618,6 +760,12 @@ template <typename VT, typename XT, bool UPPER>
 void sweep_groups(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaStream_t s, const int *gate)
 {
     const int nc = (int)F.colour_groups.size() - 1;
+    if (F.slices) {
+        static_assert(std::is_same<VT, XT>::value, "factor and vector types agree");
+        launch_lv<VT, UPPER>(F, status, x, y, s, gate);
+        SENK_LAUNCH_CHECK();
+        return;
+    }
     if (F.compact) {
 #define SENK_COMPACT_CASE(BS)                                                      \
     case BS:                                                                       \
@@ -782,37 +930,40 @@ void IluPlan<VT>::build(int N, const VT *lval, const int *lcind, const int *lrpt
         for (int p = cptr[k] * bs; p < cptr[k + 1] * bs; p++) colour_of[p] = k;
     }
     for (int k = cnum - 1; k >= 0; k--) bwd.push_back(fwd[k]);
-    // AUTO, as measured on the 128^3 system: FP32 factors on compact chains
-    // with the lanes of a chain holding its rows, one launch per colour
-    // (application 0.085 ms, against 0.139 ms with a lane per chain and 0.193
-    // ms on row slots), FP64 factors on row slots (0.303 ms against 0.318 ms
-    // row-per-lane and 0.405 ms lane-per-chain). COLOURS: row slots; COMPACT:
-    // compact chains per colour, a lane per chain; ROWS: a chain's rows in its
-    // lanes; DATAFLOW: compact chains, one launch per sweep. A factor whose
-    // widest group does not fit shared memory falls back to row slots.
+    // AUTO, as measured on the 128^3 system: FP64 factors on row-sorted slices,
+    // one launch per colour (k_sweep_lv: 0.154 ms per application, against
+    // 0.302 ms on row slots and 0.317 ms row per lane); FP32 factors on compact
+    // chains with the lanes of a chain holding its rows (0.085 ms, against
+    // 0.110 ms on slices, 0.139 ms with a lane per chain and 0.193 ms on row
+    // slots). COLOURS: row slots; COMPACT: compact chains per colour, a lane
+    // per chain; ROWS: a chain's rows in its lanes; DATAFLOW: compact chains,
+    // one launch per sweep. A factor whose groups do not fit shared memory
+    // falls back to row slots.
     const bool persistent = sweep_mode == SENK_SWEEP_PERSISTENT;
+    const bool slices = sweep_mode == SENK_SWEEP_AUTO && sizeof(VT) == 8;
     const bool rows = sweep_mode == SENK_SWEEP_ROWS || sweep_mode == SENK_SWEEP_ROWS_WIDE ||
-                      (sweep_mode == SENK_SWEEP_AUTO && sizeof(VT) == 4);
+                      (sweep_mode == SENK_SWEEP_AUTO && !slices);
     const bool wide = sweep_mode == SENK_SWEEP_WIDE || sweep_mode == SENK_SWEEP_ROWS_WIDE;
     const bool compact = sweep_mode == SENK_SWEEP_COMPACT || sweep_mode == SENK_SWEEP_DATAFLOW || persistent || wide ||
-                         rows || (sweep_mode == SENK_SWEEP_AUTO && sizeof(VT) == 4);
+                         rows;
     const bool df = sweep_mode == SENK_SWEEP_DATAFLOW;
-    if (!(compact && build_factor_wf(L, false, N, lval, lcind, lrptr, fwd, bs, colour_of, df, s, nullptr, rows)))
-        build_factor(L, false, N, lval, lcind, lrptr, fwd, nullptr, bs, &colour_of, s);
-    else {
-        L.persistent = persistent;
-        L.force_wide = wide;
-        shape_wf_bs<VT, false>(L);
-    }
+    auto build_one = [&](SweepFactor<VT> &F, auto upper, const VT *v, const int *c, const int *r,
+                         const std::vector<Group> &colours) {
+        constexpr bool kUpper = decltype(upper)::value;
+        if (slices && build_factor_lv<VT, kUpper>(F, N, v, c, r, colours, bs, colour_of, s)) {
+            shape_lv<VT, kUpper>(F);
+        } else if (compact && build_factor_wf(F, kUpper, N, v, c, r, colours, bs, colour_of, df, s, nullptr, rows)) {
+            F.persistent = persistent;
+            F.force_wide = wide;
+            shape_wf_bs<VT, kUpper>(F);
+        } else {
+            build_factor(F, kUpper, N, v, c, r, colours, nullptr, bs, &colour_of, s);
+        }
+    };
+    build_one(L, std::false_type{}, lval, lcind, lrptr, fwd);
     // For U, "earlier" means a later colour: flip the colour numbers.
     for (int p = 0; p < N; p++) colour_of[p] = cnum - 1 - colour_of[p];
-    if (!(compact && build_factor_wf(U, true, N, uval, ucind, urptr, bwd, bs, colour_of, df, s, nullptr, rows)))
-        build_factor(U, true, N, uval, ucind, urptr, bwd, nullptr, bs, &colour_of, s);
-    else {
-        U.persistent = persistent;
-        U.force_wide = wide;
-        shape_wf_bs<VT, true>(U);
-    }
+    build_one(U, std::true_type{}, uval, ucind, urptr, bwd);
 }
 
 template <typename VT>
