@@ -147,9 +147,9 @@ struct SpmvOp {
 int csr_lanes(long long nnz, int n);
 
 void launch_spmv_csr_d(const double *v, const int *c, const int *r, const double *x, const double *b,
-                       double *y, int n, int lanes, int mode, cudaStream_t s, const int *gate);
+                       double *y, int n, long long nnz, int lanes, int mode, cudaStream_t s, const int *gate);
 void launch_spmv_csr_s(const float *v, const int *c, const int *r, const float *x, const float *b,
-                       float *y, int n, int lanes, int mode, cudaStream_t s, const int *gate);
+                       float *y, int n, long long nnz, int lanes, int mode, cudaStream_t s, const int *gate);
 
 // ----------------------------------------------------------- ILU sweeps
 

@@ -83,6 +83,144 @@ k_spmv_csr(const MT *__restrict__ val, const int *__restrict__ cind, const int *
     }
 }
 
+// sum += v[u] * xv[u] for the last n of 8 slots (n the same in the whole warp).
+// FP64 enters the chain by a jump, in order (a predicated FP64 instruction
+// costs as much as one that runs, see sub_last); FP32 adds into four sums.
+template <typename T, int S>
+__device__ __forceinline__ void add_last8(T (&sum)[S], const T (&v)[8], const T (&xv)[8], int n)
+{
+    if constexpr (S == 1) {
+        switch (n) {
+        case 8: sum[0] += v[0] * xv[0];
+        case 7: sum[0] += v[1] * xv[1];
+        case 6: sum[0] += v[2] * xv[2];
+        case 5: sum[0] += v[3] * xv[3];
+        case 4: sum[0] += v[4] * xv[4];
+        case 3: sum[0] += v[5] * xv[5];
+        case 2: sum[0] += v[6] * xv[6];
+        case 1: sum[0] += v[7] * xv[7];
+        default: break;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 8; u++) sum[u % S] += v[u] * xv[u];
+    }
+}
+
+// 16 bytes global -> shared without registers; bytes past `valid` are zeroed
+// and not read.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid) : "memory");
+}
+
+// CSR SpMV of short rows: one warp takes 32 consecutive rows at a time, whose
+// entries are consecutive, copies them to shared memory (cp.async, 16 bytes a
+// lane, the next 32 rows' while these are added), and every lane adds one row
+// with its x gathers issued eight at a time. Neighbouring rows have
+// neighbouring columns, so a gather of 32 rows falls in few sectors.
+//
+// FP64 is why: the unit takes one warp instruction in 19 cycles per SM, and
+// G lanes per row (k_spmv_csr) spend log2(G) additions for 32 / G rows besides
+// the products; here a warp's FP64 instructions are its 32 rows' longest row.
+// Rows are added in column order in FP64 and into four sums in FP32 (one
+// running sum would round more than the lanes did).
+//
+// 7-point rows: FP64 128^3 158 -> 41 us (5.3 TB/s), FP32 128^3 59 -> 30 us
+// (4.8 TB/s); 27-point rows on 96^3 FP64 345 -> 89 us, FP32 95 -> 49 us (before:
+// k_spmv_csr). Its copies and sums share the SM with 32 warps, so what is left
+// is FP64's 28 us and the bytes' 32 us at 128^3 not overlapping entirely.
+//
+// val and cind 16-byte aligned. cap: entries a buffer holds (a multiple of 4);
+// 32 rows with more take several rounds. MODE 0: y = A x; MODE 1: y = b - A x.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(128, 8)
+k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const int *__restrict__ rptr,
+                const T *__restrict__ x, const T *__restrict__ b, T *__restrict__ y, int n, int cap, const int *gate)
+{
+    if (gated(gate)) return;
+    constexpr int S = sizeof(T) == 4 ? 4 : 1;
+    constexpr int EV = 16 / (int)sizeof(T);  // entries of a 16-byte piece of val
+    extern __shared__ __align__(16) unsigned char csr[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const size_t one = (size_t)(cap + 4) * (sizeof(T) + 4);  // a buffer: values, columns
+    unsigned char *buf = csr + 2 * one * wib;
+    const int step = gridDim.x * (blockDim.x >> 5), tiles = (n + 31) >> 5;
+    int tile = blockIdx.x * (blockDim.x >> 5) + wib;
+    if (tile >= tiles) return;
+    const int nnz = __ldg(rptr + n);
+    auto bounds = [&](int t, int &a, int &e) {
+        const int r = t * 32 + lane;
+        a = t < tiles ? __ldg(rptr + min(r, n)) : 0;
+        e = t < tiles ? __ldg(rptr + min(r + 1, n)) : 0;
+    };
+    // entries [c0, c0 + cap) of the tile that ends at s1 into buffer k; c0 is
+    // rounded down to a multiple of 4
+    auto fetch = [&](int k, int c0, int s1) {
+        T *sv = reinterpret_cast<T *>(buf + k * one);
+        int *sc = reinterpret_cast<int *>(sv + cap + 4);
+        const int cnt = min(cap, s1 - c0);
+        for (int i = lane * EV; i < cnt; i += 32 * EV)
+            cp_async16(sv + i, val + c0 + i, min(16, (nnz - c0 - i) * (int)sizeof(T)));
+        for (int i = lane * 4; i < cnt; i += 128) cp_async16(sc + i, cind + c0 + i, min(16, (nnz - c0 - i) * 4));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int a, e, a1, e1, k = 0;
+    bounds(tile, a, e);
+    bounds(tile + step, a1, e1);
+    int c0 = __shfl_sync(0xffffffffu, a, 0) & ~3, s1 = __shfl_sync(0xffffffffu, e, 31);
+    fetch(0, c0, s1);
+    T sum[S] = {};
+    for (;;) {
+        // the next round: the rest of this tile, or the next tile
+        const bool more = c0 + cap < s1;
+        int d0 = c0 + cap, t1 = s1;
+        if (!more) {
+            d0 = __shfl_sync(0xffffffffu, a1, 0) & ~3;
+            t1 = __shfl_sync(0xffffffffu, e1, 31);
+        }
+        const bool any = more || tile + step < tiles;
+        if (any) fetch(k ^ 1, d0, t1);
+        if (any) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        const T *sv = reinterpret_cast<const T *>(buf + k * one);
+        const int *sc = reinterpret_cast<const int *>(sv + cap + 4);
+        const int lo = max(a - c0, 0), len = min(e - c0, cap) - lo;
+        const int longest = __reduce_max_sync(0xffffffffu, len);
+        for (int k0 = 0; k0 < longest; k0 += 8) {
+            const int m = min(8, longest - k0), f = k0 - (8 - m);
+            T v[8], xv[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                v[u] = T(0);
+                xv[u] = T(0);
+                if (f + u >= k0 && f + u < len) {
+                    xv[u] = __ldg(x + sc[lo + f + u]);
+                    v[u] = sv[lo + f + u];
+                }
+            }
+            add_last8<T, S>(sum, v, xv, m);
+        }
+        __syncwarp();  // buffer k may be filled again
+        if (!more) {
+            const int row = tile * 32 + lane;
+            if constexpr (S == 4) sum[0] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            if (row < n) y[row] = MODE == 1 ? b[row] - sum[0] : sum[0];
+#pragma unroll
+            for (int u = 0; u < S; u++) sum[u] = T(0);
+            tile += step;
+            if (tile >= tiles) return;
+            a = a1;
+            e = e1;
+            bounds(tile + step, a1, e1);
+        }
+        c0 = d0;
+        s1 = t1;
+        k ^= 1;
+    }
+}
+
 // Row sum of one SELL-32 row (lane r of the slice at element offset o, w
 // columns): sum over k of val * x[col] in column order. The entries are taken
 // eight at a time with every load of a batch issued before the first product
