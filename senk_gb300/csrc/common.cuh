@@ -122,6 +122,13 @@ __device__ __forceinline__ void named_bar(int id, int nthreads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// Arrival at barrier `id` of `nthreads` threads without waiting for it (the
+// other threads wait by named_bar).
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
 // One bulk copy global -> shared (both 16-byte aligned, bytes a multiple of 16);
 // completion is counted on `bar`.
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)

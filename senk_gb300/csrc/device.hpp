@@ -177,9 +177,13 @@ struct SweepFactor {
     std::vector<int> colour_slots; // compact: widest block of each colour
     DevBuf<unsigned char> wcounts; // compact: per chain, external and in-chain counts of each row
     DevBuf<int> dcolour_groups;    // compact: colour_groups on the device
-    DevBuf<int4> levels;           // compact, per colour: {first group, groups, first slot, slots}
-    DevBuf<VT> cdinv;              // compact U: inverted diagonal per chain (small systems)
-    size_t level_bytes = 0;        // compact, chains of one row: most bytes one colour stages
+    // compact, chains of one row: a block per colour, the blocks' descriptors
+    // and batches (SmallFactor), most bytes of a block
+    DevBuf<int4> levels;
+    DevBuf<int2> batches;
+    std::vector<int4> host_levels;
+    DevBuf<unsigned char> blocks;
+    size_t level_bytes = 0;
     // compact, per colour: the launches of a sweep in order
     struct Launch {
         int g0, g1;        // groups of the colour
@@ -227,7 +231,10 @@ struct IluPlan {
     DevBuf<int> status;  // non-zero after a sweep whose bounded wait ran out (1: flag, 2: TMA)
     // small systems (the vector fits in shared memory): both sweeps in one CTA
     bool small = false;
-    int small_threads = 0;
+    int small_threads = 0, small_sets = 1;
+    bool small_fast = false;
+    auto small_kernel() const -> void (*)(SmallFactor, SmallFactor, int, const VT *, VT *, int, const int *, int *,
+                                          int, int);
     size_t small_buf = 0;          // bytes of each staging buffer
     int small_nbuf = 2;            // staging buffers (levels staged ahead + 1)
     void sweep_small(int which, const VT *x, VT *y, cudaStream_t s, const int *gate) const;

@@ -961,66 +961,93 @@ k_sweep(const GroupDesc *__restrict__ groups, int g_begin, const unsigned char *
     if (live) y[row] = tsh[l][q];
 }
 
+// t -= v[u] * yy[u] for the last n of B slots (1 <= n <= B; n the same in the
+// whole warp), in order. The entry into the chain is a jump: this chip runs an
+// FP64 instruction in about 19 cycles per SM (one unit, one warp instruction
+// at a time), and a predicated one costs the same when all of its lanes are
+// off (measured: 65 cycles a step in one warp either way), so slots without
+// an entry must not be issued.
+template <int B, typename VT, typename XT>
+__device__ __forceinline__ void sub_last(XT &t, const VT (&v)[B], const XT (&yy)[B], int n)
+{
+    static_assert(B == 3 || B == 6, "batches of three or six");
+    switch (n) {
+    case 6: if constexpr (B == 6) t -= (XT)v[B - 6] * yy[B - 6];
+    case 5: if constexpr (B == 6) t -= (XT)v[B - 5] * yy[B - 5];
+    case 4: if constexpr (B == 6) t -= (XT)v[B - 4] * yy[B - 4];
+    case 3: t -= (XT)v[B - 3] * yy[B - 3];
+    case 2: t -= (XT)v[B - 2] * yy[B - 2];
+    case 1: t -= (XT)v[B - 1] * yy[B - 1];
+    default: break;
+    }
+}
+
 // ------------------------------------------------- small systems, one CTA
 // One triangular factor in the compact chain layout, chains of one row (level
-// sets of the natural order, or AMC colours), for k_ilu_small.
-template <typename VT>
+// sets of the natural order, or AMC colours), for k_ilu_small. The data of a
+// level (colour) is one block: the groups, 32 chain descriptors per group, the
+// groups' column words and values and, for U, 32 inverted diagonals per group.
+// Consecutive levels are staged together, a batch by one bulk copy.
 struct SmallFactor {
-    const WfGroup *groups;
-    const int2 *chains;
-    const VT *val;
-    const int *col;
-    const VT *cdinv;        // U: inverted diagonal per chain
-    const int4 *levels;     // per colour (level set), processing order: {first group, groups, first slot, slots}
-    int ncolours;
+    const unsigned char *blocks;
+    const int4 *levels;   // per level, processing order: {place, groups, first slot, slots}, place =
+                          // 16-byte unit within its batch | kSmallFirst | batch << 16
+    const int2 *batches;  // {first 16-byte unit, units}
+    int ncolours, nbatches;
 };
+constexpr int kSmallFirst = 0x8000;  // the level is its batch's first
 
-// Stages the data of one level (colour) lv into buf with bulk copies counted on
-// bar: group descriptors, chain descriptors, the groups' blocks (columns, then
-// values) and, for U, the chains' inverted diagonals. One thread; no global
-// loads, so a stage costs the issuing thread a few instructions.
+// Bytes of a level's block.
 template <typename VT>
-__device__ __forceinline__ void small_stage(const SmallFactor<VT> &F, bool upper, int4 lv, unsigned char *buf,
-                                            unsigned long long *bar)
+SENK_HD constexpr unsigned small_level_bytes(int groups, int slots, bool upper)
 {
-    const int g0 = lv.x, G = lv.y, e0 = lv.z, ne = lv.w;
-    const unsigned bytes = G > 0 ? (unsigned)G * 16u + (unsigned)G * 256u + (unsigned)ne * (4u + (unsigned)sizeof(VT)) +
-                                       (upper ? (unsigned)G * 32u * (unsigned)sizeof(VT) : 0u)
-                                 : 0u;
-    // earlier generic accesses to this buffer come before the async writes
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(bar, bytes);
-    if (G == 0) return;
-    unsigned char *p = buf;
-    bulk_g2s(p, F.groups + g0, (unsigned)G * 16u, bar);
-    p += G * 16;
-    bulk_g2s(p, F.chains + (size_t)g0 * 32, (unsigned)G * 256u, bar);
-    p += G * 256;
-    if (ne > 0) {
-        bulk_g2s(p, F.col + e0, (unsigned)ne * 4u, bar);
-        p += (size_t)ne * 4;
-        bulk_g2s(p, F.val + e0, (unsigned)ne * (unsigned)sizeof(VT), bar);
-        p += (size_t)ne * sizeof(VT);
-    }
-    if (upper) bulk_g2s(p, F.cdinv + (size_t)g0 * 32, (unsigned)G * 32u * (unsigned)sizeof(VT), bar);
+    return (unsigned)groups * (16u + 256u + (upper ? 32u * (unsigned)sizeof(VT) : 0u)) +
+           (unsigned)slots * (4u + (unsigned)sizeof(VT));
 }
 
 // Both triangular sweeps of one ILU application y = U^-1 L^-1 x for a system
 // whose vector fits in shared memory, in one CTA (which: bit 0 L, bit 1 U;
 // x == y allowed). The levels (colours) run in order, one consumer thread per
-// row, with a barrier among the consumers between levels. The last warp stages:
-// its first lane copies each level's data by TMA into one of nbuf buffers (2 to
-// 8) as soon as the consumers have released that buffer (full / empty
-// mbarriers per buffer), so up to nbuf levels are in flight ahead of the one
-// being solved and no staging work lies on the consumers' path. A wait that
-// runs out sets *status = 2 and a shared abort flag; the other side stops at
-// its next wait, and the stager waits (bounded) for every copy it issued
-// before it leaves.
+// row. The last warp stages: its first lane copies each batch of levels by TMA
+// into one of nbuf buffers (2 to 8) as soon as the consumers have released
+// that buffer (full / empty mbarriers per buffer); a copy per level would take
+// it about 500 cycles a level, longer than the level itself.
+//
+// What bounds it is the chain of levels (255 per triangle for the natural
+// order of a 128 x 128 grid, about 64 rows each), so only what depends on the
+// level before lies on it. SETS = 2 or 4: that many sets of consumers take the
+// levels in turn; while one solves a level the others read their next level's
+// rows, columns and values into registers, and a set hands over to the next by
+// a barrier that it only arrives at. A level then costs the barrier, one round
+// of shared-memory reads and the row's dependent FP64 instructions (65 cycles
+// each here). SETS = 1: one set of up to 992 threads, for levels with more
+// rows than half of the CTA holds. nbuf >= SETS: a set that waits for its next
+// level's batch may then rely on the buffer's batch before that having landed.
+// FAST: no row has more than three entries and no level more rows than a set.
+// Natural order of 2D Poisson 128^2, one application: FP64 0.119 ms, FP32 0.057 ms
+// (one set that read the level's data after the barrier: 0.291 and 0.270 ms).
+//
+// A wait that runs out sets *status = 2 and a shared abort flag; every wait
+// gives up once it sees the flag, consumers still pass all barriers, and the
+// stager waits (bounded) for every copy it issued before it leaves.
 constexpr int kSmallMaxBufs = 8;
 
-template <typename VT, typename XT>
+// Wait for phase `parity` of `bar` that gives up when *flag is set, and sets it
+// (and *status) when it runs out of polls.
+__device__ __forceinline__ bool small_wait(unsigned long long *bar, unsigned parity, int *flag, int *status)
+{
+    for (unsigned i = 0; i < kWaitLimit; i++) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (*(volatile int *)flag) return false;
+    }
+    atomicExch(status, 2);
+    *(volatile int *)flag = 1;
+    return false;
+}
+
+template <typename VT, typename XT, int SETS, bool FAST>
 __global__ void __launch_bounds__(1024)
-k_ilu_small(SmallFactor<VT> Lf, SmallFactor<VT> Uf, int which, const XT *x, XT *y, int n, const int *gate,
+k_ilu_small(SmallFactor Lf, SmallFactor Uf, int which, const XT *x, XT *y, int n, const int *gate,
             int *status, int buf_bytes, int nbuf)
 {
     extern __shared__ __align__(128) unsigned char sms[];
@@ -1029,12 +1056,13 @@ k_ilu_small(SmallFactor<VT> Lf, SmallFactor<VT> Uf, int which, const XT *x, XT *
     if (gated(gate)) return;
     const int nl = (which & 1) ? Lf.ncolours : 0, nu = (which & 2) ? Uf.ncolours : 0, steps = nl + nu;
     // shared memory: the vector, the descriptors of all levels in processing
-    // order (copied once, so the stager reads no global memory between levels),
-    // then the staging buffers (small_smem_bytes)
+    // order, then the staging buffers (small_smem_bytes)
+    const int nbl = (which & 1) ? Lf.nbatches : 0, nb = nbl + ((which & 2) ? Uf.nbatches : 0);
     XT *ysh = reinterpret_cast<XT *>(sms);
-    int4 *lvs = reinterpret_cast<int4 *>(sms + ((size_t)n * sizeof(XT) + 127) / 128 * 128);
+    int4 *lvs = reinterpret_cast<int4 *>(sms + ((size_t)(n + 2) * sizeof(XT) + 127) / 128 * 128);
     unsigned char *bufs = reinterpret_cast<unsigned char *>(lvs) + ((size_t)steps * 16 + 127) / 128 * 128;
     const int ncons = (int)blockDim.x - 32;  // consumer threads; the last warp stages
+    const int ns = ncons / SETS;             // threads of a set
     if (threadIdx.x == 0) {
         for (int b = 0; b < nbuf; b++) {
             mbar_init(&full[b], 1);
@@ -1042,87 +1070,126 @@ k_ilu_small(SmallFactor<VT> Lf, SmallFactor<VT> Uf, int which, const XT *x, XT *
         }
         abort_flag = 0;
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ysh[i] = x[i];
-    for (int j = threadIdx.x; j < steps; j += blockDim.x)
-        lvs[j] = j < nl ? __ldg(Lf.levels + j) : __ldg(Uf.levels + (j - nl));
+    for (int i = threadIdx.x; i < n + 2; i += blockDim.x) ysh[i] = i < n ? x[i] : XT(0);
+    for (int j = threadIdx.x; j < steps; j += blockDim.x) {
+        int4 lv = j < nl ? __ldg(Lf.levels + j) : __ldg(Uf.levels + (j - nl));
+        const int q = (lv.x >> 16) + (j < nl ? 0 : nbl);  // batch; its buffer and the parity of its fill instead
+        lv.x = (lv.x & 0xffff) | (q % nbuf) << 16 | (q / nbuf & 1) << 24;
+        lvs[j] = lv;
+    }
     __syncthreads();
     if ((int)threadIdx.x >= ncons) {
         if ((int)threadIdx.x != ncons) return;
-        // stager: step j fills buffer b = j % nbuf for its (j / nbuf)-th time
+        // stager: batch q fills buffer b = q % nbuf for its (q / nbuf)-th time
         int issued = 0;
         unsigned epar = 0u;  // bit b: parity of buffer b's next release
-        for (int j = 0, b = 0; j < steps; j++, b = b + 1 == nbuf ? 0 : b + 1) {
-            if (j >= nbuf) {  // released by the consumers after step j - nbuf
+        auto batch = [&](int q) {
+            return q < nbl ? __ldg(Lf.batches + q) : q < nb ? __ldg(Uf.batches + (q - nbl)) : make_int2(0, 0);
+        };
+        int2 ahead = batch(0);
+        for (int q = 0, b = 0; q < nb; q++, b = b + 1 == nbuf ? 0 : b + 1) {
+            if (q >= nbuf) {  // released by the consumers after batch q - nbuf
                 const unsigned par = (epar >> b) & 1u;
                 epar ^= 1u << b;
-                bool got = false;
-                for (unsigned i = 0; i < kWaitLimit && !got; i++) {
-                    got = mbar_try_wait(&empty[b], par);
-                    if (!got && *(volatile int *)&abort_flag) break;
-                }
-                if (!got) {
-                    if (!*(volatile int *)&abort_flag) {
-                        atomicExch(status, 2);
-                        *(volatile int *)&abort_flag = 1;
-                    }
-                    break;
-                }
+                if (!small_wait(&empty[b], par, &abort_flag, status)) break;
             }
-            unsigned char *buf = bufs + (size_t)b * buf_bytes;
-            if (j < nl) small_stage(Lf, false, lvs[j], buf, &full[b]);
-            else small_stage(Uf, true, lvs[j], buf, &full[b]);
-            issued = j + 1;
+            const int2 bt = ahead;
+            ahead = batch(q + 1);
+            // earlier generic accesses to this buffer come before the async writes
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_expect_tx(&full[b], (unsigned)bt.y * 16u);
+            if (bt.y > 0)
+                bulk_g2s(bufs + (size_t)b * buf_bytes, (q < nbl ? Lf.blocks : Uf.blocks) + (size_t)bt.x * 16,
+                         (unsigned)bt.y * 16u, &full[b]);
+            issued = q + 1;
         }
         // the last use of each buffer: complete (consumed or not) before the CTA leaves
-        for (int j = issued > nbuf ? issued - nbuf : 0; j < issued; j++)
-            mbar_wait_bounded(&full[j % nbuf], (unsigned)(j / nbuf) & 1u, kWaitLimit);
+        for (int q = issued > nbuf ? issued - nbuf : 0; q < issued; q++)
+            mbar_wait_bounded(&full[q % nbuf], (unsigned)(q / nbuf) & 1u, kWaitLimit);
         return;
     }
-    // consumers: one barrier per level. A wait that runs out sets the abort
-    // flag (and *status = 2) before the level's barrier; after it every
-    // consumer sees the flag and all leave together.
-    unsigned fpar = 0u;  // bit b: parity of buffer b's next fill
-    for (int k = 0, b = 0; k < steps; k++, b = b + 1 == nbuf ? 0 : b + 1) {
+    constexpr int K = 3;  // entries of a row held in registers (the last ones)
+    const int set = SETS > 1 ? (int)threadIdx.x / ns : 0, tid = (int)threadIdx.x - set * ns, lane = tid & 31;
+    for (int k = set; k < steps; k += SETS) {
+        // the level's data, while the levels before are being solved
         const bool upper = k >= nl;
-        const bool ok = mbar_wait_bounded(&full[b], (fpar >> b) & 1u, kWaitLimit);
-        fpar ^= 1u << b;
-        if (!ok) {
-            atomicExch(status, 2);
-            *(volatile int *)&abort_flag = 1;
-        }
-        if (ok && !*(volatile int *)&abort_flag) {
-            const int4 lv = lvs[k];
-            const int G = lv.y, e0 = lv.z, ne = lv.w;
-            const unsigned char *sb = bufs + (size_t)b * buf_bytes;
-            const WfGroup *sd = reinterpret_cast<const WfGroup *>(sb);
-            const int2 *sc = reinterpret_cast<const int2 *>(sb + G * 16);
-            const int *scol = reinterpret_cast<const int *>(sb + G * 16 + G * 256);
-            const VT *sval = reinterpret_cast<const VT *>(sb + G * 16 + G * 256 + (size_t)ne * 4);
-            const VT *sdinv = reinterpret_cast<const VT *>(sb + G * 16 + G * 256 + (size_t)ne * (4 + sizeof(VT)));
-            for (int t = threadIdx.x; t < G * 32; t += ncons) {
-                const int gi = t >> 5, lane = t & 31;
-                const WfGroup d = sd[gi];
-                if (lane >= d.nchains) continue;
-                const int2 ch = sc[t];
-                const int row = ch.x, E = ch.y & 0xffff;
-                const int base = d.off - e0 + lane;
-                XT tt = ysh[row];
-                for (int e = 0; e < E; e++) tt -= (XT)sval[base + e * 32] * ysh[scol[base + e * 32] & kColMask];
-                if (upper) tt *= (XT)sdinv[t];
-                ysh[row] = tt;
+        const int4 lv = lvs[k];
+        const int b = lv.x >> 16 & 255;
+        const bool ok = small_wait(&full[b], (unsigned)lv.x >> 24, &abort_flag, status);
+        const int G = lv.y, e0 = lv.z, ne = lv.w;
+        const unsigned char *sb = bufs + (size_t)b * buf_bytes + (lv.x & (kSmallFirst - 1)) * 16;
+        const WfGroup *sd = reinterpret_cast<const WfGroup *>(sb);
+        const int2 *sc = reinterpret_cast<const int2 *>(sb + G * 16);
+        const int *scol = reinterpret_cast<const int *>(sb + G * 16 + G * 256);
+        const VT *sval = reinterpret_cast<const VT *>(sb + G * 16 + G * 256 + (size_t)ne * 4);
+        const VT *sdinv = reinterpret_cast<const VT *>(sb + G * 16 + G * 256 + (size_t)ne * (4 + sizeof(VT)));
+        // unused entries read the zero at ysh[n]; lanes without a row work on ysh[n + 1]
+        int row = n + 1, emax = 0, E = 0, base = 0, c[K];
+        VT v[K];
+        XT di = XT(1);
+        auto fetch = [&](int t) {  // the row of place t (a warp's places are one group)
+            const WfGroup d = sd[t >> 5];
+            const int2 ch = sc[t];
+            emax = d.emax;
+            base = d.off - e0 + lane;
+            const bool live = lane < d.nchains;
+            row = live ? ch.x : n + 1;
+            E = live ? ch.y & 0xffff : 0;
+            if (upper) di = (XT)sdinv[t];
+#pragma unroll
+            for (int u = 0; u < K; u++) {
+                const int e = emax - K + u;
+                c[u] = n;
+                v[u] = VT(0);
+                if (e >= 0 && e < E) {
+                    c[u] = scol[base + e * 32] & kColMask;
+                    v[u] = sval[base + e * 32];
+                }
             }
-        }
-        named_bar(1, ncons);  // the level's rows are final and buffer b is free
-        if (*(volatile int *)&abort_flag) return;
-        if (threadIdx.x == 0) mbar_arrive(&empty[b]);
+        };
+        auto solve = [&]() {
+            XT t = ysh[row], yy[K];
+#pragma unroll
+            for (int u = 0; u < K; u++) yy[u] = ysh[c[u]];
+            if (!FAST) {
+#pragma unroll 1
+                for (int e = 0; e < emax - K; e++)
+                    if (e < E) t -= (XT)sval[base + e * 32] * ysh[scol[base + e * 32] & kColMask];
+            }
+            if constexpr (sizeof(XT) == 8) {
+                sub_last<K>(t, v, yy, FAST ? emax : min(emax, K));
+                if (upper) t *= di;
+            } else {  // FP32: unused entries subtract 0 * 0, L's rows are multiplied by one
+#pragma unroll
+                for (int u = 0; u < K; u++) t -= (XT)v[u] * yy[u];
+                t *= di;
+            }
+            if (row < n) ysh[row] = t;
+        };
+        const bool mine = ok && tid - lane < G * 32;
+        if (mine) fetch(tid);
+        if (SETS > 1 && k > 0) named_bar(1 + k % SETS, 2 * ns);  // the level before is solved
+        if (mine) solve();
+        if (!FAST && ok)
+            for (int t = tid + ns; t - lane < G * 32; t += ns) {
+                fetch(t);
+                solve();
+            }
+        if (SETS == 1) named_bar(1, ncons);
+        else if (k + 1 < steps) named_bar_arrive(1 + (k + 1) % SETS, 2 * ns);
+        // this set's first thread has seen the level before end: its batch is
+        // consumed if this level starts the next one
+        if (tid == 0 && k > 0 && (lv.x & kSmallFirst)) mbar_arrive(&empty[b == 0 ? nbuf - 1 : b - 1]);
     }
+    named_bar(1 + SETS, ncons);
     for (int i = threadIdx.x; i < n; i += ncons) y[i] = ysh[i];
 }
 
-// Dynamic shared memory of k_ilu_small: vector, level descriptors, buffers.
+// Dynamic shared memory of k_ilu_small: vector (and two spare places), level
+// descriptors, buffers.
 inline size_t small_smem_bytes(size_t n, size_t xt_bytes, int steps, size_t buf_bytes, int nbuf)
 {
-    return (n * xt_bytes + 127) / 128 * 128 + ((size_t)steps * 16 + 127) / 128 * 128 + (size_t)nbuf * buf_bytes;
+    return ((n + 2) * xt_bytes + 127) / 128 * 128 + ((size_t)steps * 16 + 127) / 128 * 128 + (size_t)nbuf * buf_bytes;
 }
 
 // ------------------------------------------------------ dataflow sweeps
@@ -1920,27 +1987,6 @@ k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (live[r]) y[row[r]] = a[r].out();
-}
-
-// t -= v[u] * yy[u] for the last n of B slots (1 <= n <= B; n the same in the
-// whole warp), in order. The entry into the chain is a jump: this chip runs an
-// FP64 instruction in about 19 cycles per SM (one unit, one warp instruction
-// at a time), and a predicated one costs the same when all of its lanes are
-// off (measured: 65 cycles a step in one warp either way), so slots without
-// an entry must not be issued.
-template <int B, typename VT, typename XT>
-__device__ __forceinline__ void sub_last(XT &t, const VT (&v)[B], const XT (&yy)[B], int n)
-{
-    static_assert(B == 3 || B == 6, "batches of three or six");
-    switch (n) {
-    case 6: if constexpr (B == 6) t -= (XT)v[B - 6] * yy[B - 6];
-    case 5: if constexpr (B == 6) t -= (XT)v[B - 5] * yy[B - 5];
-    case 4: if constexpr (B == 6) t -= (XT)v[B - 4] * yy[B - 4];
-    case 3: t -= (XT)v[B - 3] * yy[B - 3];
-    case 2: t -= (XT)v[B - 2] * yy[B - 2];
-    case 1: t -= (XT)v[B - 1] * yy[B - 1];
-    default: break;
-    }
 }
 
 // Resident CTAs per SM that k_sweep_lv is compiled for: 40 registers a thread.

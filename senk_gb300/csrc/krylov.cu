@@ -119,7 +119,7 @@ void System<T>::create(const senk_system_desc &d, const senk_options *o, cudaStr
     if (pc) {
         for (const SweepFactor<T> *F : {&pc->L, &pc->U})
             h2d_bytes += (long long)(F->val.bytes() + F->col.bytes() + F->dinv.bytes() + F->rowmap.bytes() +
-                                     F->groups.bytes() + F->widths.bytes() + F->lblocks.bytes());
+                                     F->groups.bytes() + F->widths.bytes() + F->lblocks.bytes() + F->blocks.bytes());
     }
     if (d.mixed) {
         SENK_REQUIRE(sizeof(T) == sizeof(double), "mixed precision needs an FP64 system");

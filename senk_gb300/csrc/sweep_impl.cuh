@@ -209,7 +209,8 @@ constexpr size_t kSmallSmem = 220 * 1024;
 template <typename VT>
 bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const int *cind, const int *rptr,
                      const std::vector<Group> &colours, int bs, const std::vector<int> &colour_of, bool dataflow,
-                     cudaStream_t s, const std::vector<int> *rowmap = nullptr, bool chain_major = false)
+                     cudaStream_t s, const std::vector<int> *rowmap = nullptr, bool chain_major = false,
+                     bool one_cta = false)
 {
     std::vector<WfColour> cr;
     for (const Group &g : colours) cr.push_back({g.p0, g.p1});
@@ -235,6 +236,37 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.colour_groups = lay.colour_groups;
     F.colour_slots = lay.colour_slots;
     F.colour_smem.assign(F.colour_slots.size(), 0);
+    if (one_cta) {  // each level's data as one block, for k_ilu_small
+        F.level_bytes = 0;
+        std::vector<int4> lv;
+        std::vector<unsigned char> blocks;
+        blocks.reserve(lay.groups.size() * (272 + (upper ? 32 * sizeof(VT) : 0)) + lay.col.size() * (4 + sizeof(VT)));
+        auto put = [&](const auto *p, size_t count) {
+            const unsigned char *q = reinterpret_cast<const unsigned char *>(p);
+            blocks.insert(blocks.end(), q, q + count * sizeof(*p));
+        };
+        for (size_t c = 0; c + 1 < lay.colour_groups.size(); c++) {
+            const int g0 = lay.colour_groups[c], g1 = lay.colour_groups[c + 1];
+            int e0 = 0, ne = 0;
+            if (g1 > g0) {
+                const WfGroup &last = lay.groups[g1 - 1];
+                e0 = lay.groups[g0].off;
+                ne = last.off + (last.emax + last.imax) * 32 - e0;
+            }
+            lv.push_back(make_int4((int)(blocks.size() / 16), g1 - g0, e0, ne));  // x: unit in the blocks
+            put(lay.groups.data() + g0, (size_t)(g1 - g0));
+            put(lay.chains.data() + (size_t)g0 * 32, (size_t)(g1 - g0) * 32);
+            put(lay.col.data() + e0, (size_t)ne);
+            put(lay.val.data() + e0, (size_t)ne);
+            if (upper) put(lay.cdinv.data() + (size_t)g0 * 32, (size_t)(g1 - g0) * 32);
+            F.level_bytes = std::max<size_t>(F.level_bytes, small_level_bytes<VT>(g1 - g0, ne, upper));
+        }
+        F.host_levels = std::move(lv);
+        F.blocks.alloc(std::max<size_t>(blocks.size(), 16));
+        F.blocks.upload(blocks.data(), blocks.size(), s);
+        SENK_CUDA(cudaStreamSynchronize(s));
+        return true;
+    }
     F.val.alloc(std::max<size_t>(lay.val.size(), 1));
     F.val.upload(lay.val.data(), lay.val.size(), s);
     F.col.alloc(std::max<size_t>(lay.col.size(), 1));
@@ -251,33 +283,6 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.wcounts.upload(lay.counts.data(), lay.counts.size(), s);
     F.dcolour_groups.alloc(lay.colour_groups.size());
     F.dcolour_groups.upload(lay.colour_groups.data(), lay.colour_groups.size(), s);
-    std::vector<int4> lv;
-    for (size_t c = 0; c + 1 < lay.colour_groups.size(); c++) {
-        const int g0 = lay.colour_groups[c], g1 = lay.colour_groups[c + 1];
-        int e0 = 0, ne = 0;
-        if (g1 > g0) {
-            const WfGroup &last = lay.groups[g1 - 1];
-            e0 = lay.groups[g0].off;
-            ne = last.off + (last.emax + last.imax) * 32 - e0;
-        }
-        lv.push_back(make_int4(g0, g1 - g0, e0, ne));
-    }
-    F.levels.alloc(std::max<size_t>(lv.size(), 1));
-    F.levels.upload(lv.data(), lv.size(), s);
-    if (upper) {
-        F.cdinv.alloc(std::max<size_t>(lay.cdinv.size(), 1));
-        F.cdinv.upload(lay.cdinv.data(), lay.cdinv.size(), s);
-    }
-    F.level_bytes = 0;
-    for (size_t c = 0; c + 1 < lay.colour_groups.size(); c++) {
-        const int G = lay.colour_groups[c + 1] - lay.colour_groups[c];
-        long long ne = 0;
-        for (int g = lay.colour_groups[c]; g < lay.colour_groups[c + 1]; g++)
-            ne += (long long)(lay.groups[g].emax + lay.groups[g].imax) * 32;
-        const size_t b = (size_t)G * 16 + (size_t)G * 256 + (size_t)ne * (4 + sizeof(VT)) +
-                         (upper ? (size_t)G * 32 * bs * sizeof(VT) : 0);
-        F.level_bytes = std::max(F.level_bytes, b);
-    }
     if (!dataflow) {
         // one launch per colour; x is read early from the second colour on
         const int nc = (int)lay.colour_groups.size() - 1;
@@ -812,20 +817,29 @@ void allow_all_smem()
 
 }  // namespace
 
+// The form of k_ilu_small that fits the plan's levels.
+template <typename VT>
+auto IluPlan<VT>::small_kernel() const -> void (*)(SmallFactor, SmallFactor, int, const VT *, VT *, int, const int *,
+                                                   int *, int, int)
+{
+    if (small_sets == 4) return small_fast ? k_ilu_small<VT, VT, 4, true> : k_ilu_small<VT, VT, 4, false>;
+    if (small_sets == 2) return small_fast ? k_ilu_small<VT, VT, 2, true> : k_ilu_small<VT, VT, 2, false>;
+    return k_ilu_small<VT, VT, 1, false>;
+}
+
 template <typename VT>
 void IluPlan<VT>::sweep_small(int which, const VT *x, VT *y, cudaStream_t s, const int *gate) const
 {
     auto mk = [](const SweepFactor<VT> &F) {
-        return SmallFactor<VT>{(const WfGroup *)F.wgroups.p, (const int2 *)F.wchains.p, (const VT *)F.val.p,
-                               (const int *)F.col.p, (const VT *)F.cdinv.p, (const int4 *)F.levels.p,
-                               (int)F.colour_groups.size() - 1};
+        return SmallFactor{(const unsigned char *)F.blocks.p, (const int4 *)F.levels.p, (const int2 *)F.batches.p,
+                           (int)F.colour_groups.size() - 1, (int)F.batches.n};
     };
     const int steps = ((which & 1) ? (int)L.colour_groups.size() - 1 : 0) +
                       ((which & 2) ? (int)U.colour_groups.size() - 1 : 0);
     const size_t smem = small_smem_bytes((size_t)n, sizeof(VT), steps, small_buf, small_nbuf);
-    // small_threads consumers and one staging warp
-    k_ilu_small<VT, VT><<<1, small_threads + 32, smem, s>>>(mk(L), mk(U), which, x, y, n, gate, status.p,
-                                                            (int)small_buf, small_nbuf);
+    // small_threads consumers (in one, two or four sets) and one staging warp
+    auto kern = small_kernel();
+    kern<<<1, small_threads + 32, smem, s>>>(mk(L), mk(U), which, x, y, n, gate, status.p, (int)small_buf, small_nbuf);
     SENK_LAUNCH_CHECK();
 }
 
@@ -862,23 +876,54 @@ void IluPlan<VT>::build_small(int N, const VT *lval, const int *lcind, const int
         }
         for (int k = cnum - 1; k >= 0; k--) gu.push_back(gl[k]);
     }
-    if (!build_factor_wf(L, false, N, lval, lcind, lrptr, gl, bs, col_l, false, s, rml.empty() ? nullptr : &rml))
+    if (!build_factor_wf(L, false, N, lval, lcind, lrptr, gl, bs, col_l, false, s, rml.empty() ? nullptr : &rml, false,
+                         true))
         return;
-    if (!build_factor_wf(U, true, N, uval, ucind, urptr, gu, bs, col_u, false, s, rmu.empty() ? nullptr : &rmu))
+    if (!build_factor_wf(U, true, N, uval, ucind, urptr, gu, bs, col_u, false, s, rmu.empty() ? nullptr : &rmu, false, true))
         return;
     int most = 32;
     for (const SweepFactor<VT> *F : {&L, &U})
         for (size_t c = 0; c + 1 < F->colour_groups.size(); c++)
             most = std::max(most, (F->colour_groups[c + 1] - F->colour_groups[c]) * 32);
-    small_threads = std::min(992, (most + 31) / 32 * 32);
-    small_buf = (std::max(L.level_bytes, U.level_bytes) + 127) / 128 * 128;
-    // the vector and the descriptors of both factors' levels (one application)
+    // the vector and the descriptors of both factors' levels (one application);
+    // what is left in six buffers, or as many as hold the largest level
     const int steps = (int)L.colour_groups.size() - 1 + (int)U.colour_groups.size() - 1;
     const size_t fixed = small_smem_bytes((size_t)N, sizeof(VT), steps, 0, 0);
-    if (fixed + 2 * small_buf > kSmallSmem) return;  // a level too large to stage next to the vector
-    small_nbuf = (int)std::min<size_t>(kSmallMaxBufs, (kSmallSmem - fixed) / std::max<size_t>(small_buf, 128));
+    const size_t level = (std::max(L.level_bytes, U.level_bytes) + 127) / 128 * 128;
+    if (fixed + 2 * level > kSmallSmem) return;  // a level too large to stage next to the vector
+    small_buf = std::max<size_t>({level, std::min<size_t>((kSmallSmem - fixed) / 6, 16 * 1024) / 128 * 128, 128});
+    small_nbuf = (int)std::min<size_t>(kSmallMaxBufs, (kSmallSmem - fixed) / small_buf);
+    for (SweepFactor<VT> *F : {&L, &U}) {
+        std::vector<int2> batches;
+        std::vector<int4> lv = F->host_levels;
+        for (size_t c = 0; c < lv.size(); c++) {
+            const int u0 = F->host_levels[c].x,
+                      u1 = c + 1 < lv.size() ? F->host_levels[c + 1].x : (int)(F->blocks.n / 16);
+            if (batches.empty() || (size_t)(u1 - batches.back().x) * 16 > small_buf) {
+                batches.push_back(make_int2(u0, 0));
+                lv[c].x = kSmallFirst;
+            } else {
+                lv[c].x = u0 - batches.back().x;
+            }
+            lv[c].x |= (int)(batches.size() - 1) << 16;
+            batches.back().y = u1 - batches.back().x;
+        }
+        if (batches.size() > 32767) return;
+        F->levels.alloc(lv.size());
+        F->levels.upload(lv.data(), lv.size(), s);
+        F->batches.alloc(batches.size());
+        F->batches.upload(batches.data(), batches.size(), s);
+        SENK_CUDA(cudaStreamSynchronize(s));
+    }
+    // four or two sets while a set holds the widest level; with more rows than
+    // that the rounds over a level's rows weigh more than the hand-over
+    small_sets = most <= 240 && small_nbuf > 4 ? 4 : most <= 480 ? 2 : 1;
+    small_threads = small_sets > 1 ? small_sets * most : std::min(992, most);
     const size_t smem = small_smem_bytes((size_t)N, sizeof(VT), steps, small_buf, small_nbuf);
-    SENK_CUDA(cudaFuncSetAttribute(k_ilu_small<VT, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    small_fast = small_sets > 1;
+    for (int i = 0; i < N; i++)
+        small_fast = small_fast && lrptr[i + 1] - lrptr[i] <= 3 && urptr[i + 1] - urptr[i] <= 4;
+    SENK_CUDA(cudaFuncSetAttribute(small_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     small = true;
 }
 
