@@ -281,6 +281,25 @@ struct IlubPlan {
     DevBuf<int2> chains;               // (first block row, block rows)
     std::vector<int> phase_chains;     // chain range of each phase
     long long lblocks = 0, ublocks = 0;
+    // ABMC, chains of up to 16 block rows: the factors in slices of block rows
+    // (k_ilub_slices) instead of the BCSR arrays
+    bool sliced = false;
+    int per = 0;                       // block rows per chain
+    struct Slices {
+        struct Launch {
+            int g0, g1;      // groups of the colour
+            int early_x;     // 1: x is read before the wait on the previous kernel
+            size_t smem = 0;
+        };
+        std::vector<Launch> launches;  // in processing order
+        DevBuf<int4> groups;           // BlGroup
+        DevBuf<T> ext;                 // external values
+        DevBuf<unsigned char> blob;    // staged parts
+    };
+    Slices ls, us;
+    DevBuf<int> status;                // non-zero after a staging wait that ran out
+    bool build_slices(bool upper, const int *bcind, const int *brptr, const std::vector<int2> &ch, cudaStream_t s);
+    void check_status(cudaStream_t s) const;
 
     void build(int N, int bnl, int bnw, const T *blval, const int *blcind, const int *blrptr, const T *buval,
                const int *bucind, const int *burptr, const int *cptr, int cnum, int bsize, cudaStream_t s);
@@ -293,8 +312,8 @@ struct IlubPlan {
     long long apply_bytes() const;
     long long h2d_bytes() const
     {
-        return (long long)(lval.bytes() + uval.bytes() + lcind.bytes() + lrptr.bytes() + ucind.bytes() +
-                           urptr.bytes() + chains.bytes());
+        const long long bs = (long long)bnl * bnw;
+        return (lblocks + ublocks) * (bs * (long long)sizeof(T) + 4) + 2LL * (nbr + 1) * 4 + (long long)chains.bytes();
     }
 };
 

@@ -130,6 +130,287 @@ k_ilub_sweep(const T *__restrict__ bval, const int *__restrict__ bcind, const in
     }
 }
 
+
+// ------------------------------------------------ ABMC: slices of block rows
+// Chains of one colour, RPW = 32 / BNL (rounded down) to a group: lane
+// g * BNL + r holds row r of chain g's block row in every phase, and step q of
+// a group is the q-th block row of its chains. A block row's blocks outside its
+// chain (rows of earlier colours, which come first in the reference's order)
+// are its external slots, the others its in-chain slots; a step is as wide as
+// its widest block row (padding: column -1, value 0).
+struct BlGroup {
+    int row0;  // first block row
+    int nch;   // chains
+    int ext;   // first external slot (BNW * 32 values each)
+    int blob;  // first 16-byte unit of the staged part
+};
+
+constexpr int kBlMaxSteps = 16;
+
+// Byte offsets of a group's staged part: widths (external, in-chain) of each
+// step, the external block columns, the in-chain columns (scalar, from the
+// chain's first row), the in-chain values and U's diagonal squares.
+struct BlParts {
+    unsigned cols, lc, val, diag, end;
+};
+__host__ __device__ inline BlParts bl_parts(int per, int we, int wi, int rpw, int bnl, int bnw, bool upper, unsigned vb)
+{
+    auto up = [](unsigned b) { return (b + 15u) / 16u * 16u; };
+    BlParts p;
+    p.cols = up(4u * per);
+    p.lc = p.cols + up(4u * we * rpw);
+    p.val = p.lc + up(4u * wi * rpw);
+    p.diag = p.val + 32u * vb * wi * bnw;
+    p.end = p.diag + (upper ? 32u * vb * per * bnl : 0u);
+    return p;
+}
+
+// Fills a group's external values and staged part from the BCSR factor. One
+// CTA per group, warp q = step q.
+template <typename T, int BNL, int BNW, bool UPPER>
+__global__ void __launch_bounds__(32 * kBlMaxSteps)
+k_ilub_fill(const BlGroup *__restrict__ groups, const uint16_t *__restrict__ widths, int per, int nbr,
+            const T *__restrict__ bval, const int *__restrict__ bcind, const int *__restrict__ brptr, T *ext,
+            unsigned char *blob)
+{
+    constexpr int RPW = 32 / BNL, BS = BNL * BNW, BREM = BNL / BNW;
+    const BlGroup d = groups[blockIdx.x];
+    const uint16_t *wd = widths + (size_t)blockIdx.x * 2 * per;
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / BNL, r = lane % BNL;
+    int we0 = 0, wi0 = 0, we = 0, wi = 0;
+    for (int k = 0; k < per; k++) {
+        if (k == q) {
+            we0 = we;
+            wi0 = wi;
+        }
+        we += wd[k];
+        wi += wd[per + k];
+    }
+    const BlParts P = bl_parts(per, we, wi, RPW, BNL, BNW, UPPER, sizeof(T));
+    unsigned char *t = blob + (size_t)d.blob * 16;
+    if (lane == 0) {
+        reinterpret_cast<uint16_t *>(t)[q] = wd[q];
+        reinterpret_cast<uint16_t *>(t)[per + q] = wd[per + q];
+    }
+    int *cols = reinterpret_cast<int *>(t + P.cols), *lc = reinterpret_cast<int *>(t + P.lc);
+    T *val = reinterpret_cast<T *>(t + P.val), *diag = reinterpret_cast<T *>(t + P.diag);
+    T *xv = ext + (size_t)d.ext * BNW * 32;
+    const int br = d.row0 + g * per + q, first = (d.row0 + g * per) * BNL, last = first + per * BNL;
+    const bool live = g < RPW && g < d.nch && br < nbr;
+    int ke = 0, ki = 0;
+    if (live) {
+        const int a = brptr[br] + (UPPER ? BREM : 0), e = brptr[br + 1];
+        for (int i = a; i < e; i++) {
+            const int j = UPPER ? e - 1 - (i - a) : i;
+            const int c = bcind[j] * BNW;
+            const bool in = c >= first && c < last;
+            T *to = in ? val + (size_t)(wi0 + ki) * BNW * 32 : xv + (size_t)(we0 + ke) * BNW * 32;
+            for (int l = 0; l < BNW; l++) to[l * 32 + lane] = bval[(size_t)j * BS + l * BNL + r];
+            if (r == 0) {
+                if (in) lc[(wi0 + ki) * RPW + g] = c - first;
+                else cols[(we0 + ke) * RPW + g] = bcind[j];
+            }
+            if (in) ki++;
+            else ke++;
+        }
+    }
+    for (; ke < wd[q]; ke++) {
+        for (int l = 0; l < BNW; l++) xv[((size_t)(we0 + ke) * BNW + l) * 32 + lane] = T(0);
+        if (r == 0 && g < RPW) cols[(we0 + ke) * RPW + g] = -1;
+    }
+    for (; ki < wd[per + q]; ki++) {
+        for (int l = 0; l < BNW; l++) val[((size_t)(wi0 + ki) * BNW + l) * 32 + lane] = T(0);
+        if (r == 0 && g < RPW) lc[(wi0 + ki) * RPW + g] = -1;
+    }
+    if (UPPER)
+        for (int c = 0; c < BNL; c++)  // column c of the diagonal square
+            diag[((size_t)q * BNL + c) * 32 + lane] =
+                live ? bval[(size_t)(brptr[br] + c / BNW) * BS + (c % BNW) * BNL + r] : T(0);
+}
+
+// t -= v[k][l] * gy[k][l] over the last n of 4 slots, in order (n the same in
+// the whole warp); the entry is a jump, see sub_last.
+template <int BNW, typename T>
+__device__ __forceinline__ void sub_slots(T &t, const T (&v)[4][BNW], const T *gy, int stride, int n)
+{
+    auto slot = [&](int k) {
+#pragma unroll
+        for (int l = 0; l < BNW; l++) t -= v[k][l] * gy[k * stride + l];
+    };
+    switch (n) {
+    case 4: slot(0);
+    case 3: slot(1);
+    case 2: slot(2);
+    case 1: slot(3);
+    default: break;
+    }
+}
+
+// One colour per launch, one CTA per group: the block rows of earlier colours
+// that the group's external slots name are gathered into shared memory, warp q
+// subtracts the external slots of step q (their values read straight into
+// registers, four slots ahead), and one warp runs the in-chain part step by
+// step, as k_ilub_sweep does. The staged part (TMA), the first external values
+// and, with early_x, x and the gate are read before the wait on the previous
+// kernel. Same operations in the same order as k_ilub_sweep, which walked a
+// chain's block rows one after another with a dependent gather per four blocks.
+// Block-3x3 system, 48^3 nodes (8 colours), one application: FP64 0.524 ->
+// 0.177 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
+// row's up to 69 FP64 subtractions at 65 cycles, then four in-chain steps) and
+// by the FP64 unit (50 us of the 177).
+template <typename T, int BNL, int BNW, bool UPPER>
+__global__ void __launch_bounds__(256)
+k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const T *__restrict__ ext,
+              const uint4 *__restrict__ blob, const T *x, T *y, const int *gate, int *status, int early_x)
+{
+    constexpr int RPW = 32 / BNL, B = 4;
+    extern __shared__ __align__(128) unsigned char bls[];
+    __shared__ __align__(8) unsigned long long bar;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
+    const int g = lane / BNL, r = lane % BNL;
+    const BlGroup d = groups[g0 + blockIdx.x], d1 = groups[g0 + blockIdx.x + 1];
+    const unsigned bytes = (unsigned)(d1.blob - d.blob) * 16u;
+    const int we = d1.ext - d.ext;  // external slots
+    const int r0 = d.row0 * BNL, nrows = min(d.nch * per * BNL, n - r0);
+    T *ysh = reinterpret_cast<T *>(bls + bytes);  // the group's rows
+    T *gy = ysh + RPW * kBlMaxSteps * BNL;        // external operands, slot after slot
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, bytes);
+        bulk_g2s(bls, blob + d.blob, bytes, &bar);
+    }
+    bool skip = false;
+    if (early_x) {
+        for (int i = tid; i < nrows; i += nt) ysh[i] = x[r0 + i];
+        skip = gated(gate);
+    } else {
+        pdl_launch_dependents();
+    }
+    __syncthreads();
+    const bool ok = mbar_wait_bounded(&bar, 0, kWaitLimit);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(status, 2);
+        if (!ok) mbar_wait_bounded(&bar, 0, kWaitLimit);
+        pdl_wait();
+        return;
+    }
+    const uint16_t *wd = reinterpret_cast<const uint16_t *>(bls);
+    int wi = 0, s0 = 0;  // in-chain slots; external slots before step w
+    for (int k = 0; k < per; k++) {
+        wi += wd[per + k];
+        if (k < w) s0 += wd[k];
+    }
+    const BlParts P = bl_parts(per, we, wi, RPW, BNL, BNW, UPPER, sizeof(T));
+    const int *cols = reinterpret_cast<const int *>(bls + P.cols);
+    const int *lc = reinterpret_cast<const int *>(bls + P.lc);
+    const T *val = reinterpret_cast<const T *>(bls + P.val), *diag = reinterpret_cast<const T *>(bls + P.diag);
+    // external values of step q: up to B slots ending at slot k1 of the step
+    T v[B][BNW];
+    auto load = [&](int first, int k1) {
+#pragma unroll
+        for (int u = 0; u < B; u++)
+            if (k1 - B + u >= 0)
+#pragma unroll
+                for (int l = 0; l < BNW; l++)
+                    v[u][l] = ld_stream(ext + ((size_t)(d.ext + first + k1 - B + u) * BNW + l) * 32 + lane);
+    };
+    int q = w, width = q < per ? wd[q] : 0, k1 = width > 0 ? (width - 1) % B + 1 : 0;
+    if (k1 > 0) load(s0, k1);
+    pdl_wait();  // the previous colour (or the producer of x) has finished
+    if (early_x) {
+        pdl_launch_dependents();
+    } else {
+        skip = gated(gate);
+        for (int i = tid; i < nrows; i += nt) ysh[i] = x[r0 + i];
+    }
+    if (skip) return;
+    for (int i = tid; i < we * RPW * BNW; i += 4 * nt) {
+        T a[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int at = i + u * nt, c = at < we * RPW * BNW ? cols[at / BNW] : -1;
+            a[u] = c >= 0 ? y[c * BNW + at % BNW] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i + u * nt < we * RPW * BNW) gy[i + u * nt] = a[u];
+    }
+    __syncthreads();
+    const int at = min(g, RPW - 1);  // lanes past the last chain repeat one; they store nothing
+    for (; q < per; q += nw) {
+        const int row = (at * per + q) * BNL + r;
+        T t = row < nrows ? ysh[row] : T(0);
+        while (k1 > 0) {
+            const int m = min(k1, B);
+            T cur[B][BNW];
+#pragma unroll
+            for (int u = 0; u < B; u++)
+#pragma unroll
+                for (int l = 0; l < BNW; l++) cur[u][l] = v[u][l];
+            const T *gk = gy + ((s0 + k1 - B) * RPW + at) * BNW;  // used from the first slot in use on
+            const int next = k1 + B;
+            if (k1 < width) load(s0, next);
+            sub_slots<BNW>(t, cur, gk, RPW * BNW, m);
+            k1 = k1 < width ? next : 0;
+        }
+        if (g < RPW && row < nrows) ysh[row] = t;
+        if (q + nw < per) {
+            for (int k = q; k < q + nw; k++) s0 += wd[k];
+            width = wd[q + nw];
+            k1 = width > 0 ? (width - 1) % B + 1 : 0;
+            if (k1 > 0) load(s0, k1);
+        }
+    }
+    __syncthreads();
+    if (w == 0) {
+        const int base = at * BNL;
+        for (int st = 0; st < per; st++) {
+            const int qq = UPPER ? per - 1 - st : st;
+            int i0 = 0;
+            for (int k = 0; k < qq; k++) i0 += wd[per + k];
+            const int row = (at * per + qq) * BNL + r;
+            const bool live = g < RPW && row < nrows;
+            T t = live ? ysh[row] : T(0);
+            const int m = wd[per + qq];
+#pragma unroll 1
+            for (int k = 0; k < m; k++) {
+                const int c = lc[(i0 + k) * RPW + at], rel0 = c - qq * BNL;
+                const bool inside = !UPPER && c >= 0 && rel0 >= 0 && rel0 < BNL;
+                const bool any = !UPPER && __any_sync(0xffffffffu, inside);
+#pragma unroll
+                for (int l = 0; l < BNW; l++) {
+                    const T vv = val[((size_t)(i0 + k) * BNW + l) * 32 + lane];
+                    const T yy = c >= 0 ? ysh[at * per * BNL + c + l] : T(0);
+                    T tout = t;
+                    if (!any || __any_sync(0xffffffffu, !inside && c >= 0)) tout = t - vv * yy;
+                    if (any) {
+                        const int rel = inside ? rel0 + l : 0;
+                        const T a0 = __shfl_sync(0xffffffffu, t, base + rel);
+                        const T t0 = t - vv * a0;
+                        const T a1 = __shfl_sync(0xffffffffu, t0, base + rel);  // y[col] after its own pair
+                        const T t1 = (r >> 1) > (rel >> 1) ? t - vv * a1 : t0;
+                        if (inside) tout = t1;
+                    }
+                    t = tout;
+                }
+            }
+            if (UPPER) {
+#pragma unroll
+                for (int c = BNL - 1; c >= 0; c--) {
+                    const T dc = diag[((size_t)qq * BNL + c) * 32 + lane];
+                    if (r == c) t *= dc;
+                    const T a = __shfl_sync(0xffffffffu, t, base + c);
+                    if (r < c) t -= dc * a;
+                }
+            }
+            if (live) ysh[row] = t;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < nrows; i += nt) y[r0 + i] = ysh[i];
+}
+
 #define SENK_ILUB_SHAPES(X) X(1, 1) X(2, 1) X(2, 2) X(3, 3) X(4, 1) X(4, 2) X(4, 4) X(8, 1) X(8, 2)
 
 bool shape_supported(int bnl, int bnw)
@@ -237,6 +518,8 @@ void IlubPlan<T>::build(int N, int bnl_, int bnw_, const T *blval, const int *bl
     lblocks = blrptr[nbr];
     ublocks = burptr[nbr];
     const size_t bs = (size_t)bnl * bnw;
+    status.alloc(1);
+    SENK_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), s));
     auto put = [s](auto &buf, const auto *h, size_t count) {
         buf.alloc(count);
         buf.upload(h, count, s);
@@ -247,13 +530,152 @@ void IlubPlan<T>::build(int N, int bnl_, int bnw_, const T *blval, const int *bl
     put(uval, buval, (size_t)ublocks * bs);
     put(ucind, bucind, (size_t)ublocks);
     put(urptr, burptr, (size_t)nbr + 1);
-    put(chains, ch.data(), ch.size());
+    per = cptr ? bsize / bnl : 0;
+    sliced = cptr && per <= kBlMaxSteps && build_slices(false, blcind, blrptr, ch, s) &&
+             build_slices(true, bucind, burptr, ch, s);
+    if (!sliced) {
+        ls = Slices();
+        us = Slices();
+    }
+    if (sliced) {  // the slices hold everything the sweeps read
+        SENK_CUDA(cudaStreamSynchronize(s));
+        for (auto *v : {&lval, &uval}) v->release();
+        for (auto *v : {&lcind, &lrptr, &ucind, &urptr}) v->release();
+    } else {
+        put(chains, ch.data(), ch.size());
+    }
     SENK_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
+}
+
+// Groups, widths and the slice layout of one factor (k_ilub_slices), filled on
+// the device from the BCSR arrays uploaded before. False when a group does not
+// fit the shared memory or a block row's blocks outside its chain do not come
+// first.
+template <typename T>
+bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, const std::vector<int2> &ch,
+                               cudaStream_t s)
+{
+    const int rpw = 32 / bnl, brem = bnl / bnw;
+    const int P = (int)phase_chains.size() - 1;
+    Slices &F = upper ? us : ls;
+    std::vector<BlGroup> gd;
+    F.launches.clear();
+    for (int pi = 0; pi < P; pi++) {  // colours in processing order
+        const int p = upper ? P - 1 - pi : pi;
+        const int before = (int)gd.size();
+        for (int c = phase_chains[p]; c < phase_chains[p + 1]; c += rpw)
+            gd.push_back({ch[c].x, std::min(rpw, phase_chains[p + 1] - c), 0, 0});
+        if ((int)gd.size() > before) F.launches.push_back({before, (int)gd.size(), 0});
+    }
+    const int ng = (int)gd.size();
+    std::vector<uint16_t> widths((size_t)ng * 2 * per, 0);
+    bool fits = true;
+#pragma omp parallel for schedule(static) reduction(&& : fits)
+    for (int g = 0; g < ng; g++)
+        for (int c = 0; c < gd[g].nch; c++)
+            for (int q = 0; q < per; q++) {
+                const int br = gd[g].row0 + c * per + q, first = (gd[g].row0 + c * per) * bnl;
+                if (br >= nbr) continue;
+                int we = 0, wi = 0;
+                const int a = brptr[br] + (upper ? brem : 0), e = brptr[br + 1];
+                for (int i = a; i < e; i++) {  // in the sweep's order
+                    const int col = bcind[upper ? e - 1 - (i - a) : i] * bnw;
+                    if (col >= first && col < first + per * bnl) {
+                        wi++;
+                    } else {
+                        we++;
+                        fits = fits && wi == 0;  // external blocks come first
+                    }
+                }
+                uint16_t *w = &widths[(size_t)g * 2 * per];
+                fits = fits && we < 65536 && wi < 65536;
+                w[q] = (uint16_t)std::max<int>(w[q], we);
+                w[per + q] = (uint16_t)std::max<int>(w[per + q], wi);
+            }
+    if (!fits) return false;
+    long long ext = 0, blob = 0;
+    std::vector<size_t> smem(ng);
+    for (int g = 0; g < ng; g++) {
+        const uint16_t *w = &widths[(size_t)g * 2 * per];
+        int we = 0, wi = 0;
+        for (int q = 0; q < per; q++) {
+            we += w[q];
+            wi += w[per + q];
+        }
+        const BlParts parts = bl_parts(per, we, wi, rpw, bnl, bnw, upper, sizeof(T));
+        gd[g].ext = (int)ext;
+        gd[g].blob = (int)blob;
+        ext += we;
+        blob += parts.end / 16;
+        smem[g] = parts.end + ((size_t)rpw * kBlMaxSteps * bnl + (size_t)we * rpw * bnw) * sizeof(T);
+        if (smem[g] > 160 * 1024 || ext >= (1 << 30) || blob >= (1 << 30)) return false;
+    }
+    gd.push_back({0, 0, (int)ext, (int)blob});
+    size_t most = 48 * 1024;
+    for (size_t k = 0; k < F.launches.size(); k++) {
+        auto &L = F.launches[k];
+        L.early_x = k > 0;
+        for (int g = L.g0; g < L.g1; g++) L.smem = std::max(L.smem, smem[g]);
+        most = std::max(most, L.smem);
+    }
+    F.groups.alloc(gd.size());
+    F.groups.upload((const int4 *)gd.data(), gd.size(), s);
+    F.ext.alloc(std::max<size_t>((size_t)ext * bnw * 32, 1));
+    F.blob.alloc(std::max<size_t>((size_t)blob * 16, 16));
+    DevBuf<uint16_t> dw(widths.size());
+    dw.upload(widths.data(), widths.size(), s);
+    const BlGroup *dg = (const BlGroup *)F.groups.p;
+#define X(R, C)                                                                                                  \
+    if (bnl == R && bnw == C) {                                                                                  \
+        if (upper) {                                                                                             \
+            k_ilub_fill<T, R, C, true><<<ng, 32 * per, 0, s>>>(dg, dw.p, per, nbr, uval.p, ucind.p, urptr.p, F.ext.p, \
+                                                               F.blob.p);                                        \
+            SENK_CUDA(cudaFuncSetAttribute(k_ilub_slices<T, R, C, true>,                                         \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));             \
+        } else {                                                                                                 \
+            k_ilub_fill<T, R, C, false><<<ng, 32 * per, 0, s>>>(dg, dw.p, per, nbr, lval.p, lcind.p, lrptr.p,    \
+                                                                F.ext.p, F.blob.p);                              \
+            SENK_CUDA(cudaFuncSetAttribute(k_ilub_slices<T, R, C, false>,                                        \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));             \
+        }                                                                                                        \
+    } else
+    SENK_ILUB_SHAPES(X)
+#undef X
+    throw ArgError("unsupported ILUB block shape");
+    SENK_LAUNCH_CHECK();
+    SENK_CUDA(cudaStreamSynchronize(s));  // the widths go out of scope
+    return true;
 }
 
 template <typename T>
 void IlubPlan<T>::sweep(bool upper, const T *x, T *y, cudaStream_t s, const int *gate) const
 {
+    if (sliced) {
+        const Slices &F = upper ? us : ls;
+        for (const auto &L : F.launches) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(L.g1 - L.g0);
+            cfg.blockDim = dim3(32 * std::min(per, 8));
+            cfg.dynamicSmemBytes = L.smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+#define X(R, C)                                                                                                \
+    if (bnl == R && bnw == C)                                                                                  \
+        SENK_CUDA(cudaLaunchKernelEx(&cfg, upper ? k_ilub_slices<T, R, C, true> : k_ilub_slices<T, R, C, false>, \
+                                     (const BlGroup *)F.groups.p, L.g0, per, n, (const T *)F.ext.p,             \
+                                     (const uint4 *)F.blob.p, x, y, gate, status.p, L.early_x));                \
+    else
+            SENK_ILUB_SHAPES(X)
+#undef X
+            throw ArgError("unsupported ILUB block shape");
+        }
+        SENK_LAUNCH_CHECK();
+        return;
+    }
     const int P = (int)phase_chains.size() - 1;
     const int G = lanes_of(bnl);
     for (int pi = 0; pi < P; pi++) {
@@ -277,6 +699,20 @@ void IlubPlan<T>::sweep(bool upper, const T *x, T *y, cudaStream_t s, const int 
         throw ArgError("unsupported ILUB block shape");
         SENK_LAUNCH_CHECK();
     }
+}
+
+template <typename T>
+void IlubPlan<T>::check_status(cudaStream_t s) const
+{
+    int h = 0;
+    SENK_CUDA(cudaMemcpyAsync(&h, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SENK_CUDA(cudaStreamSynchronize(s));
+    if (!h) return;
+    // reported once: the next sweep starts clean
+    SENK_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), s));
+    SENK_CUDA(cudaStreamSynchronize(s));
+    throw CudaError{cudaErrorLaunchTimeout, "ILUB sweep: a TMA copy of a group's factor block did not complete", __FILE__,
+                    __LINE__};
 }
 
 template <typename T>
@@ -317,6 +753,7 @@ template <typename T>
 void System<T>::check_pc() const
 {
     if (pc) pc->check_status(stream);
+    if (pcb) pcb->check_status(stream);
 }
 
 template void System<double>::precondition(const double *, double *, const int *);

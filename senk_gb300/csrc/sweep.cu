@@ -51,6 +51,7 @@ int senk_ilu_plan_status(senk_ilu_plan *plan, void *stream)
         SENK_CUDA(cudaDeviceSynchronize());
         if (plan->d) plan->d->check_status(nullptr);
         else if (plan->f) plan->f->check_status(nullptr);
+        else if (plan->b) plan->b->check_status(nullptr);
         return (int)kOk;
     });
 }
