@@ -194,6 +194,7 @@ struct SweepFactor {
         int coop = 0, cbeg = 0, cend = 0, grid = 0;
         // 1: k_sweep_cc2 (two rows per thread) instead of k_sweep_cc
         int wide = 0;
+        int rows = 0;      // k_sweep_lv: rows per group
     };
     std::vector<Launch> launches;
     DevBuf<WfGroup> wgroups;
@@ -214,7 +215,6 @@ struct SweepFactor {
     // row-sorted slice layout, one launch per colour (k_sweep_lv): its groups
     // and their blocks; `launches` gives the colours
     bool slices = false;
-    int lv_rows = 0;               // rows per group
     DevBuf<LvGroup> lgroups;
     DevBuf<unsigned char> lblocks;
     // compact, per colour, external entries chain-major: k_sweep_rl (lanes =

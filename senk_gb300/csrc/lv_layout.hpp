@@ -115,7 +115,7 @@ struct LvLayout {
     size_t bytes = 0;
     std::vector<int> colour_groups;
     std::vector<size_t> colour_smem;  // most shared memory of a group of each colour
-    int gr = 0;                   // rows per group
+    std::vector<int> colour_rows;     // rows per group of each colour
     long long stored = 0;
 };
 
@@ -186,34 +186,38 @@ inline void lv_sort(std::vector<int> &rows, std::vector<int> &tmp, const unsigne
 }
 
 // The groups (rows only) of each colour: 512 rows each, halved while some
-// group's entries take more than `want` bytes (down to one chain or 32 rows).
-// Returns the rows per group.
-inline int lv_cut(std::vector<LvGroup> &gd, std::vector<int> &colour_groups, const int *rptr,
-                  const std::vector<std::pair<int, int>> &colours, int bs, size_t want, size_t vb)
+// group's entries take more than `want` bytes (down to one chain or 32 rows) or
+// the colour has fewer than `spread` groups (down to 64 rows).
+inline void lv_cut(std::vector<LvGroup> &gd, std::vector<int> &colour_groups, std::vector<int> &colour_rows,
+                   const int *rptr, const std::vector<std::pair<int, int>> &colours, int bs, size_t want, int spread,
+                   size_t vb)
 {
-    for (int gr = kLvMaxRows;; gr /= 2) {
-        gd.clear();
-        colour_groups.assign(1, 0);
-        size_t worst = 0;
-        for (const auto &c : colours) {
-            for (int p = c.first; p < c.second; p += gr) {
-                const int nrows = std::min(gr, c.second - p);
-                gd.push_back({p, nrows, 0, 0});
-                worst = std::max(worst, (size_t)(rptr[p + nrows] - rptr[p]) * (2 + vb));
-            }
-            colour_groups.push_back((int)gd.size());
+    gd.clear();
+    colour_groups.assign(1, 0);
+    colour_rows.clear();
+    for (const auto &c : colours) {
+        int gr = kLvMaxRows;
+        for (;; gr /= 2) {
+            size_t worst = 0;
+            for (int p = c.first; p < c.second; p += gr)
+                worst = std::max(worst, (size_t)(rptr[std::min(p + gr, c.second)] - rptr[p]) * (2 + vb));
+            const bool more = worst > want || (gr > 64 && (long long)gr * spread > c.second - c.first);
+            if (!more || gr / 2 < std::max(32, bs)) break;
         }
-        if (worst <= want || gr / 2 < std::max(32, bs)) return gr;
+        for (int p = c.first; p < c.second; p += gr) gd.push_back({p, std::min(gr, c.second - p), 0, 0});
+        colour_groups.push_back((int)gd.size());
+        colour_rows.push_back(gr);
     }
 }
 
 // Builds the layout of one factor. colour_of[row]: the colour's index in
-// processing order; `want` as for lv_cut. Throws std::invalid_argument when the factor does not fit the schedule;
+// processing order; `want` and `spread` as for lv_cut.
+// Throws std::invalid_argument when the factor does not fit the schedule;
 // returns false when a group's block would need more than `most` bytes.
 template <typename VT>
 bool make_lv_layout(LvLayout<VT> &out, bool upper, int N, const VT *val, const int *cind, const int *rptr,
                     const std::vector<std::pair<int, int>> &colours, int bs, const int *colour_of, size_t want,
-                    size_t most)
+                    int spread, size_t most)
 {
     if (bs < 1 || bs > 32 || N % bs) throw std::invalid_argument("chain length must divide N and be at most 32");
     std::vector<unsigned char> ne(N), ni(N), lev(N);
@@ -260,7 +264,7 @@ bool make_lv_layout(LvLayout<VT> &out, bool upper, int N, const VT *val, const i
     }
     if (covered != N) throw std::invalid_argument("colours do not cover the N rows");
     std::vector<LvGroup> gd;
-    const int gr = lv_cut(gd, out.colour_groups, rptr, colours, bs, want, sizeof(VT));
+    lv_cut(gd, out.colour_groups, out.colour_rows, rptr, colours, bs, want, spread, sizeof(VT));
     const int ng = (int)gd.size();
     std::vector<std::vector<unsigned char>> block(ng);
     std::vector<size_t> smem(ng);
@@ -420,7 +424,6 @@ bool make_lv_layout(LvLayout<VT> &out, bool upper, int N, const VT *val, const i
         std::vector<unsigned char>().swap(block[g]);
     }
     out.groups = std::move(gd);
-    out.gr = gr;
     out.stored = stored;
     return true;
 }

@@ -324,7 +324,11 @@ bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, 
     std::vector<std::pair<int, int>> cr;
     for (const Group &g : colours) cr.push_back({g.p0, g.p1});
     LvLayout<VT> lay;
-    lay.gr = lv_cut(lay.groups, lay.colour_groups, rptr, cr, bs, kLvWantBytes, sizeof(VT));
+    // at least two groups per SM: a narrow colour's FP64 instructions then use
+    // every SM's unit (application at 76^3 92 -> 84 us, at 48^3 80 -> 73 us;
+    // four groups per SM: 88 and 73 us)
+    const int spread = 2 * sm_count();
+    lv_cut(lay.groups, lay.colour_groups, lay.colour_rows, rptr, cr, bs, kLvWantBytes, spread, sizeof(VT));
     const int ng = (int)lay.groups.size();
     std::vector<LvJob> jobs;
     for (size_t c = 0; c < cr.size(); c++)
@@ -362,7 +366,8 @@ bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, 
     if (bad) {
         // reports a row that does not fit the schedule (throws), or builds
         // what the device builder's tables do not hold
-        if (!make_lv_layout(lay, UPPER, N, val, cind, rptr, cr, bs, colour_of.data(), kLvWantBytes, kMaxStagedBytes))
+        if (!make_lv_layout(lay, UPPER, N, val, cind, rptr, cr, bs, colour_of.data(), kLvWantBytes, spread,
+                            kMaxStagedBytes))
             return false;
         on_host = true;
     } else {
@@ -378,7 +383,6 @@ bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, 
     F.mapped = false;
     F.bs = bs;
     F.slices = true;
-    F.lv_rows = lay.gr;
     F.nnz = (long long)nnz;
     F.colour_groups = lay.colour_groups;
     F.lgroups.alloc(lay.groups.size());
@@ -398,6 +402,7 @@ bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, 
         L.g1 = lay.colour_groups[c + 1];
         L.early_x = F.launches.empty() ? 0 : 1;
         L.smem = lay.colour_smem[c];
+        L.rows = lay.colour_rows[c];
         if (L.g1 > L.g0) F.launches.push_back(L);
     }
     SENK_CUDA(cudaStreamSynchronize(s));  // the arrays used above are released on return
@@ -625,7 +630,7 @@ void launch_lv(const SweepFactor<VT> &F, int *status, const VT *x, VT *y, cudaSt
     for (const auto &L : F.launches) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(L.g1 - L.g0);
-        cfg.blockDim = dim3(L.wide ? F.lv_rows / 2 : F.lv_rows);
+        cfg.blockDim = dim3(L.wide ? L.rows / 2 : L.rows);
         cfg.dynamicSmemBytes = L.smem;
         cfg.stream = s;
         cudaLaunchAttribute at[1];
@@ -650,11 +655,11 @@ void shape_lv(SweepFactor<VT> &F)
     for (const auto &L : F.launches) most = std::max(most, L.smem);
     SENK_CUDA(cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     SENK_CUDA(cudaFuncSetAttribute(half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    if (F.lv_rows < 64) return;
     for (auto &L : F.launches) {
+        if (L.rows < 64) continue;
         int one = 0, two = 0;
-        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, full, F.lv_rows, L.smem));
-        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, half, F.lv_rows / 2, L.smem));
+        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, full, L.rows, L.smem));
+        SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, half, L.rows / 2, L.smem));
         L.wide = (L.g1 - L.g0) > one * sm_count() && two > one ? 1 : 0;
     }
 }

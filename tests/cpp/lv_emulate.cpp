@@ -12,7 +12,7 @@ namespace {
 
 template <typename VT>
 int emulate(int N, const VT *val, const int *cind, const int *rptr, int upper, const int *cptr, int cnum, int bs,
-            int want, const VT *x, VT *y, int *info, char *err, int errlen)
+            int want, int spread, const VT *x, VT *y, int *info, char *err, int errlen)
 {
     auto fail = [&](const char *m) {
         std::snprintf(err, errlen, "%s", m);
@@ -27,10 +27,10 @@ int emulate(int N, const VT *val, const int *cind, const int *rptr, int upper, c
             for (int p = cptr[c] * bs; p < cptr[c + 1] * bs; p++) colour_of[p] = k;
         }
         LvLayout<VT> L;
-        if (!make_lv_layout(L, upper != 0, N, val, cind, rptr, colours, bs, colour_of.data(), (size_t)want,
+        if (!make_lv_layout(L, upper != 0, N, val, cind, rptr, colours, bs, colour_of.data(), (size_t)want, spread,
                             (size_t)1 << 30))
             return fail("layout does not fit");
-        info[0] = L.gr;
+        info[0] = *std::min_element(L.colour_rows.begin(), L.colour_rows.end());
         std::vector<VT> yy(x, x + N);
         std::vector<int> done(N, 0);
         long long stored = 0;
@@ -41,7 +41,7 @@ int emulate(int N, const VT *val, const int *cind, const int *rptr, int upper, c
                 const unsigned char *t = L.blocks.get() + (size_t)d.off * 16;
                 const LvHeader *h = (const LvHeader *)t;
                 const LvParts P = lv_parts(*h, upper ? d.nrows * (unsigned)sizeof(VT) : 0u, sizeof(VT));
-                if (d.nrows < 1 || d.nrows > L.gr || P.end != (unsigned)d.units * 16 || ((size_t)d.off + d.units) * 16 > L.bytes ||
+                if (d.nrows < 1 || d.nrows > L.colour_rows[k] || P.end != (unsigned)d.units * 16 || ((size_t)d.off + d.units) * 16 > L.bytes ||
                     lv_smem(P.end, d.nrows, h->ncols, sizeof(VT)) > L.colour_smem[k])
                     return fail("group larger than its colour's staging buffer");
                 const uint32_t *word = (const uint32_t *)(h + 1);
@@ -136,13 +136,13 @@ int emulate(int N, const VT *val, const int *cind, const int *rptr, int upper, c
 }  // namespace
 
 extern "C" int lv_emulate_d(int N, const double *val, const int *cind, const int *rptr, int upper, const int *cptr,
-                            int cnum, int bs, int want, const double *x, double *y, int *info, char *err, int errlen)
+                            int cnum, int bs, int want, int spread, const double *x, double *y, int *info, char *err, int errlen)
 {
-    return emulate(N, val, cind, rptr, upper, cptr, cnum, bs, want, x, y, info, err, errlen);
+    return emulate(N, val, cind, rptr, upper, cptr, cnum, bs, want, spread, x, y, info, err, errlen);
 }
 
 extern "C" int lv_emulate_s(int N, const float *val, const int *cind, const int *rptr, int upper, const int *cptr,
-                            int cnum, int bs, int want, const float *x, float *y, int *info, char *err, int errlen)
+                            int cnum, int bs, int want, int spread, const float *x, float *y, int *info, char *err, int errlen)
 {
-    return emulate(N, val, cind, rptr, upper, cptr, cnum, bs, want, x, y, info, err, errlen);
+    return emulate(N, val, cind, rptr, upper, cptr, cnum, bs, want, spread, x, y, info, err, errlen);
 }

@@ -48,11 +48,12 @@ def test_emulated_slice_sweep_equals_the_oracle(emu, port, kind, n, bs, dtype):
     Ar, Lf, Uf, nc, sc = _system(kind, n, bs)
     x = np.random.default_rng(7).uniform(-1, 1, Ar.n).astype(dtype)
     f = emu.lv_emulate_s if dtype == np.float32 else emu.lv_emulate_d
-    for want in (32 * 1024, 8 * 1024):   # full groups, and groups halved to fit a small buffer
+    # full groups, groups halved to fit a small buffer, and halved to make many
+    for want, spread in ((32 * 1024, 1), (8 * 1024, 1), (32 * 1024, 100)):
         t = x
         for F, upper in ((Lf.astype(dtype), 0), (Uf.astype(dtype), 1)):
             y, err, info = np.zeros_like(t), C.create_string_buffer(256), (C.c_int * 2)()
-            rc = f(Ar.n, L.ptr(F.val), L.ptr(F.cind), L.ptr(F.rptr), upper, L.ptr(sc), nc, bs, want, L.ptr(t),
+            rc = f(Ar.n, L.ptr(F.val), L.ptr(F.cind), L.ptr(F.rptr), upper, L.ptr(sc), nc, bs, want, spread, L.ptr(t),
                    L.ptr(y), info, err, 256)
             assert rc == 0, err.value.decode()
             want_y = port.sptrsv(F, t, bool(upper))
