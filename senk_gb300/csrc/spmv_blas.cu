@@ -1,5 +1,7 @@
 // SpMV operators and the single-operation device entry points (SpMV, blas1).
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <climits>
 #include <mutex>
 
@@ -297,7 +299,32 @@ template struct SpmvOp<float>;
 namespace {
 std::mutex g_red_mu;
 ReduceScratch g_red[64];
-DevBuf<double> g_red_out[64];
+
+// The result's place in pinned host memory that the kernel writes itself, per
+// device (kept for the life of the process).
+double *g_red_host[64];
+double *g_red_host_dev[64];
+
+// A signalling NaN that no reduction returns: the place holds it until the
+// kernel has written.
+constexpr unsigned long long kNoResult = 0x7ff4a5a5c3c35a5aull;
+
+// Waits for the result of the reduction launched on s: a few hundred
+// microseconds of reading its place (a dot product of a small system takes
+// less than a copy and a synchronisation, 10 us), then the stream, whose
+// errors are reported.
+double wait_result(const double *place, cudaStream_t s)
+{
+    const volatile unsigned long long *bits = reinterpret_cast<const volatile unsigned long long *>(place);
+    const auto give_up = std::chrono::steady_clock::now() + std::chrono::microseconds(300);
+    while (*bits == kNoResult)
+        if (std::chrono::steady_clock::now() > give_up) {
+            SENK_CUDA(cudaStreamSynchronize(s));
+            break;
+        }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return *const_cast<const volatile double *>(place);
+}
 
 template <typename T, int OP>
 void elementwise(T a, T b, const T *x, T *y, T *z, int n, cudaStream_t s)
@@ -389,15 +416,17 @@ static int dev_reduce(const char *fn, const double *x, const double *y, int N, d
         cudaStream_t s = (cudaStream_t)stream;
         std::lock_guard<std::mutex> lk(g_red_mu);
         g_red[dev].ensure(s);
-        if (!g_red_out[dev].p) g_red_out[dev].alloc(1);
+        if (!g_red_host[dev]) {
+            SENK_CUDA(cudaHostAlloc((void **)&g_red_host[dev], sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
+            SENK_CUDA(cudaHostGetDevicePointer((void **)&g_red_host_dev[dev], g_red_host[dev], 0));
+        }
+        *reinterpret_cast<volatile unsigned long long *>(g_red_host[dev]) = kNoResult;
         const int grid = stream_grid(N, kThreads, 2);
         k_multidot<double, false><<<dim3(grid, 1), kThreads, 0, s>>>(x, 0, 1, y, N, g_red[dev].part.p,
-                                                                     g_red[dev].ticket.p, g_red_out[dev].p, nullptr,
+                                                                     g_red[dev].ticket.p, g_red_host_dev[dev], nullptr,
                                                                      nullptr);
         SENK_LAUNCH_CHECK();
-        double h = 0;
-        SENK_CUDA(cudaMemcpyAsync(&h, g_red_out[dev].p, sizeof(double), cudaMemcpyDeviceToHost, s));
-        SENK_CUDA(cudaStreamSynchronize(s));
+        const double h = wait_result(g_red_host[dev], s);
         *result = norm ? sqrt(h) : h;
         return (int)kOk;
     });
