@@ -272,24 +272,27 @@ k_spmv_sell32(const MT *__restrict__ val, const int *__restrict__ col, const int
 }
 
 // r = b - A x on the SELL-32 copy, with ||r||^2 reduced to the last CTA, which
-// stores ||r|| in *norm_out and 1/||r|| in *inv_out.
+// stores ||r|| in *norm_out and 1/||r|| in *inv_out. One wave of CTAs takes the
+// rows in turn: with a CTA per 256 rows the tickets and partials of 8,192 CTAs
+// took longer than the product (2.1M rows,
+// FP64 104 -> 55 us, FP32 88 -> 43 us).
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 k_residual_sell32(const T *__restrict__ val, const int *__restrict__ col, const int *__restrict__ off,
                   const int *__restrict__ perm, const T *__restrict__ x, const T *__restrict__ b,
                   T *__restrict__ r, int n, double *part, unsigned *ticket, double *norm_out, double *inv_out)
 {
     using A = typename Acc<T>::type;
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double nacc = 0;
-    if (p < n) {  // positions below n hold rows (sigma windows lie within the rows)
+    // positions below n hold rows (sigma windows lie within the rows)
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
         const int s = (int)(p >> 5), lane = (int)(p & 31);
         const int o = __ldg(off + s), w = (__ldg(off + s + 1) - o) >> 5;
         const A sum = sell_row_sum<T, T, A>(val, col, x, o, w, lane);
         const long long row = perm ? (long long)__ldg(perm + p) : p;
         const T v = (T)((A)b[row] - sum);
         r[row] = v;
-        nacc = (double)v * (double)v;
+        nacc += (double)v * (double)v;
     }
     __shared__ double sh[32];
     const double t = block_sum(nacc, sh);
@@ -791,18 +794,39 @@ inline void launch_update(int grid, cudaStream_t s, const XT *V, long long ldv, 
 }
 
 // Back-solve of the Hessenberg least squares (include/senk_blas2.hpp:24-34) for
-// the J = (converged ? jconv : m) columns of this cycle; one thread.
+// the J = (converged ? jconv : m) columns of this cycle; one warp, lane l
+// keeping rows l and l + 32 (m <= 63). A solved unknown is taken from every
+// row above it at once; each row still subtracts its columns from the last one
+// down. 30 columns: 60 -> 44 us (one thread before; most of it is FP64
+// divisions).
 static __global__ void k_gmres_trsv(KrylovState *st, const double *H, const double *e, double *y, int m)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int l = threadIdx.x;
     const int ld = m + 1;
     const int J = st->done ? st->jconv : m;
-    for (int i = J - 1; i >= 0; i--) {
-        double t = e[i];
-        for (int k = J - 1; k > i; k--) t -= H[(long long)k * ld + i] * y[k];
-        y[i] = t / H[(long long)i * ld + i];
+    double t[2], own[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; u++) t[u] = l + 32 * u < J ? e[l + 32 * u] : 0.0;
+    auto column = [&](int k, double (&h)[2]) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) h[u] = k >= 0 && l + 32 * u <= k ? H[(long long)k * ld + l + 32 * u] : 0.0;
+    };
+    double h[2], nxt[2];
+    column(J - 1, h);
+    for (int k = J - 1; k >= 0; k--) {
+        column(k - 1, nxt);  // while this column is used
+        const double tk = k < 32 ? t[0] : t[1], hk = k < 32 ? h[0] : h[1];
+        const double yk = __shfl_sync(0xffffffffu, (k & 31) == l ? tk / hk : 0.0, k & 31);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (l + 32 * u == k) own[u] = yk;
+            if (l + 32 * u < k) t[u] -= h[u] * yk;
+            h[u] = nxt[u];
+        }
     }
-    for (int i = J; i < m; i++) y[i] = 0;
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        if (l + 32 * u < m) y[l + 32 * u] = own[u];
 }
 
 // Solution update of a cycle. PRE: V0 = y0*V0 + sum_{k<J} y_k V_k (then the

@@ -273,8 +273,7 @@ void SpmvOp<T>::residual(const T *x, const T *b, T *y, ReduceScratch &red, doubl
 {
     red.ensure(s);
     if (use_sell) {
-        const int grid = ceil_div(n, kThreads);
-        SENK_REQUIRE(grid <= red.ctas * ReduceScratch::kMaxCols, "N too large for the reduction scratch");
+        const int grid = stream_grid(n, kThreads, 5);  // 48 registers a thread
         k_residual_sell32<T><<<grid, kThreads, 0, s>>>(sval.p, scol.p, soff.p, sell_perm.empty() ? nullptr : sperm.p,
                                                        x, b, y, n, red.part.p, red.ticket.p,
                                                        norm_out, inv_out);
