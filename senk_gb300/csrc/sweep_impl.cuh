@@ -281,6 +281,12 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.wchains.upload(lay.chains.data(), lay.chains.size(), s);
     F.wcounts.alloc(std::max<size_t>(lay.counts.size(), 16));
     F.wcounts.upload(lay.counts.data(), lay.counts.size(), s);
+    if (chain_major) {
+        F.wrows.alloc(std::max<size_t>(lay.rows.size(), 1));
+        F.wrows.upload(lay.rows.data(), lay.rows.size(), s);
+        F.wicol.alloc(std::max<size_t>(lay.icol.size(), 16));
+        F.wicol.upload(lay.icol.data(), lay.icol.size(), s);
+    }
     F.dcolour_groups.alloc(lay.colour_groups.size());
     F.dcolour_groups.upload(lay.colour_groups.data(), lay.colour_groups.size(), s);
     if (!dataflow) {
@@ -291,7 +297,7 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
             L.g0 = lay.colour_groups[c];
             L.g1 = lay.colour_groups[c + 1];
             L.early_x = c > 0 ? 1 : 0;
-            L.smem = ((size_t)lay.colour_slots[c] * 32 * (4 + sizeof(VT)) + 32 * 2 * (size_t)bs + 15) / 16 * 16;
+            L.smem = ((size_t)lay.colour_slots[c] * 32 * (4 + sizeof(VT)) + 32 * (chain_major ? (bs > 16 ? 8 : 4) : 2) * (size_t)bs + 15) / 16 * 16;
             if (L.g1 > L.g0) F.launches.push_back(L);
         }
     } else {
@@ -541,16 +547,17 @@ void launch_cc(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
                     cfg.blockDim = dim3(BS * 16);
                     SENK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep_rl<VT, XT, BS, UPPER, 2>, (const WfGroup *)F.wgroups.p,
                                                  L.g0, (const int2 *)F.wchains.p,
-                                                 (const unsigned char *)F.wcounts.p, (const VT *)F.val.p,
-                                                 (const int *)F.col.p, (const VT *)F.dinv.p, x, y, gate, status,
-                                                 L.early_x));
+                                                 (const unsigned *)F.wrows.p, (const VT *)F.val.p,
+                                                 (const int *)F.col.p, (const unsigned char *)F.wicol.p,
+                                                 (const VT *)F.dinv.p, x, y, gate, status, L.early_x));
                     continue;
                 }
             }
             SENK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep_rl<VT, XT, BS, UPPER, 1>, (const WfGroup *)F.wgroups.p, L.g0,
-                                         (const int2 *)F.wchains.p, (const unsigned char *)F.wcounts.p,
-                                         (const VT *)F.val.p, (const int *)F.col.p, (const VT *)F.dinv.p, x, y, gate,
-                                         status, L.early_x));
+                                         (const int2 *)F.wchains.p, (const unsigned *)F.wrows.p,
+                                         (const VT *)F.val.p, (const int *)F.col.p,
+                                         (const unsigned char *)F.wicol.p, (const VT *)F.dinv.p, x, y, gate, status,
+                                         L.early_x));
             continue;
         }
         if constexpr (BS >= 4) {
@@ -983,7 +990,7 @@ void IluPlan<VT>::build(int N, const VT *lval, const int *lcind, const int *lrpt
     // AUTO, as measured on the 128^3 system: FP64 factors on row-sorted slices,
     // one launch per colour (k_sweep_lv: 0.154 ms per application, against
     // 0.302 ms on row slots and 0.317 ms row per lane); FP32 factors on compact
-    // chains with the lanes of a chain holding its rows (0.085 ms, against
+    // chains with the lanes of a chain holding its rows (0.078 ms, against
     // 0.110 ms on slices, 0.139 ms with a lane per chain and 0.193 ms on row
     // slots). COLOURS: row slots; COMPACT: compact chains per colour, a lane
     // per chain; ROWS: a chain's rows in its lanes; DATAFLOW: compact chains,

@@ -25,7 +25,9 @@
 // streams then start in different shared-memory banks), for kernels whose
 // lanes are the rows of one chain (k_sweep_rl); the chain descriptors then
 // hold ibase_q in place of I ({first row, E | ibase_q << 16}), so that a lane
-// finds its chain's in-chain entries from its own descriptor.
+// finds its chain's in-chain entries from its own descriptor. k_sweep_rl stages
+// the column words of the external part only; it reads the in-chain columns
+// from `icol`, a byte each, and a row's counts from its row word.
 #pragma once
 
 #include <vector_functions.h>
@@ -64,11 +66,35 @@ size_t wf_bytes_for(int slots, int bs, bool upper)
            16;
 }
 
+// What a lane of k_sweep_rl needs of its row: the external entries of the
+// chain's rows solved before it (eo) and its own (ne), the same of in-chain
+// entries (io, left), and the levels of its chain. Chains of up to 16 rows take
+// one word (io <= 120 and left, depth <= 15 there), longer ones two.
+struct RowWord {
+    int eo, ne, io, left, depth;
+};
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline RowWord row_word(unsigned w)
+{
+    return {(int)(w & 1023u), (int)(w >> 10 & 127u), (int)(w >> 17 & 127u), (int)(w >> 24 & 15u), (int)(w >> 28)};
+}
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline RowWord row_word(uint2 w)
+{
+    return {(int)(w.x & 0xffffu), (int)(w.x >> 16 & 255u), (int)(w.y & 0xffffu), (int)(w.y >> 16), (int)(w.x >> 24)};
+}
+
 template <typename VT>
 struct WfLayout {
     std::vector<WfGroup> groups;  // in processing order
     std::vector<int2> chains;     // per group 32 x {first row, E | I << 16} (unused lanes {0, 0})
     std::vector<unsigned char> counts;  // per group 32 x 2*bs row counts (external, in-chain)
+    std::vector<unsigned> rows;   // chain_major: per group 32 x bs row words (row_word; two words a row for bs = 32)
+    std::vector<unsigned char> icol;  // chain_major: chain-local columns of the in-chain entries, at their places
     std::vector<VT> val;          // block values
     std::vector<int> col;         // block column words
     std::vector<VT> dinv;         // U: inverted diagonal per row
@@ -83,7 +109,8 @@ struct WfLayout {
 // Builds the layout of one factor. colour_of[row]: the colour's index in
 // processing order. Throws std::invalid_argument when the factor does not fit
 // the schedule; returns false when a group's block would need more than
-// `max_smem` bytes of shared memory per warp.
+// `max_smem` bytes of shared memory per warp, or with chain_major when a row's
+// counts do not fit its word.
 template <typename VT>
 bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const int *cind, const int *rptr,
                     const std::vector<WfColour> &colours, int bs, const int *colour_of, size_t max_smem,
@@ -181,11 +208,15 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
     out.val.assign((size_t)off, VT(0));
     out.col.assign((size_t)off, 0);
     out.counts.assign((size_t)ng * 32 * 2 * bs, 0);
+    const int rw = bs > 16 ? 2 : 1;
+    out.rows.assign(chain_major ? (size_t)ng * 32 * bs * rw : 0, 0u);
+    out.icol.assign(chain_major ? (size_t)off : 0, 0);
+    bool packs = true;
     out.cdinv.assign(upper ? (size_t)ng * 32 * bs : 0, VT(0));
     out.dinv.assign(upper ? N : 0, VT(0));
     std::vector<int> owner(N, -1);  // group of each row
     long long stored = 0;
-#pragma omp parallel for schedule(dynamic, 64) reduction(+ : stored)
+#pragma omp parallel for schedule(dynamic, 64) reduction(+ : stored) reduction(&& : packs)
     for (int g = 0; g < ng; g++) {
         const WfGroup d = gd[g];
         for (int q = 0; q < d.nchains; q++) {
@@ -193,6 +224,7 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
             int ke = 0, ki = 0;
             int ibase = 0;
             for (int q2 = 0; q2 < q; q2++) ibase += (int)((unsigned)chv[(size_t)g * 32 + q2].y >> 16);
+            int lev[32] = {};  // dependency levels of the chain's rows: 0, or 1 + the largest of the rows read
             for (int st = 0; st < bs; st++) {
                 const int l = upper ? bs - 1 - st : st;  // rows in solve order
                 const int row = r0 + l;
@@ -202,8 +234,10 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
                     const int c = cind[j];
                     if (c >= r0 && c < r0 + bs) {
                         cnt[bs + l]++;
+                        lev[l] = std::max(lev[l], lev[c - r0] + 1);
                         const long long at = d.off + (long long)d.emax * 32 + ibase + ki++;
                         out.col[at] = (l << 8) | (c - r0);
+                        if (chain_major) out.icol[at] = (unsigned char)(c - r0);
                         out.val[at] = val[j];
                     } else {
                         cnt[l]++;
@@ -222,8 +256,28 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
                     for (int j = rptr[row]; j < rptr[row + 1]; j++) put(j);
                 }
             }
+            if (chain_major) {
+                const unsigned char *cnt = out.counts.data() + ((size_t)g * 32 + q) * 2 * bs;
+                const unsigned depth = (unsigned)*std::max_element(lev, lev + bs);
+                unsigned eo = 0, io = 0;
+                for (int st = 0; st < bs; st++) {
+                    const int l = upper ? bs - 1 - st : st;
+                    const unsigned ne = cnt[l], left = cnt[bs + l];
+                    unsigned *w = &out.rows[(((size_t)g * 32 + q) * bs + l) * rw];
+                    if (rw == 1) {
+                        packs = packs && eo < 1024 && ne < 128;
+                        *w = eo | ne << 10 | io << 17 | left << 24 | depth << 28;
+                    } else {
+                        w[0] = eo | ne << 16 | depth << 24;
+                        w[1] = io | left << 16;
+                    }
+                    eo += ne;
+                    io += left;
+                }
+            }
         }
     }
+    if (!packs) return false;
     // dependencies: the groups owning each group's external columns (all earlier)
     std::vector<std::vector<int>> deps(ng);
     bad = -1;

@@ -17,7 +17,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 # (problem, n, block size): chains of 1 to 32 rows, one partly filled group,
 # rows of a dense stencil (smaller groups), several groups per colour
 CASES = [("convdiff", 16, 16), ("convdiff", 40, 16), ("convdiff", 16, 2), ("convdiff", 12, 32), ("poisson", 64, 8),
-         ("vardiff", 16, 4), ("convdiff", 12, 1), ("poisson", 200, 1), ("block", 8, 4)]
+         ("vardiff", 16, 4), ("convdiff", 12, 1), ("poisson", 200, 1), ("block", 8, 4), ("block", 8, 16),
+         ("block", 8, 32)]
 
 
 def _system(kind, n, bs):
