@@ -380,9 +380,8 @@ int senk_dev_spmv_bcsr_d(const double *bval, const int *bcind, const int *brptr,
         const int nb = N / bnl;
         if (nb == 0) return (int)kOk;
         cudaStream_t s = (cudaStream_t)stream;
-        const int grid = ceil_div(nb, kThreads);
 #define SENK_BCSR_CASE(R, C) \
-        if (bnl == R && bnw == C) { k_spmv_bcsr<double, double, R, C, 0><<<grid, kThreads, 0, s>>>(bval, bcind, brptr, x, nullptr, y, nb, nullptr); SENK_LAUNCH_CHECK(); return (int)kOk; }
+        if (bnl == R && bnw == C) { k_spmv_bcsr<double, double, R, C, 0><<<ceil_div(N, kBcsrThreads), kBcsrThreads, 0, s>>>(bval, bcind, brptr, x, nullptr, y, nb, nullptr); SENK_LAUNCH_CHECK(); return (int)kOk; }
         SENK_BCSR_CASE(1, 1) SENK_BCSR_CASE(2, 1) SENK_BCSR_CASE(2, 2) SENK_BCSR_CASE(3, 3)
         SENK_BCSR_CASE(4, 1) SENK_BCSR_CASE(4, 4) SENK_BCSR_CASE(8, 1)
 #undef SENK_BCSR_CASE
