@@ -68,21 +68,31 @@ __global__ void __launch_bounds__(kThreads) k_rms(const T *r, long long n, doubl
     }
 }
 
-// h0 = relu(f W_in + b_in), one thread per (node, feature); X0[:, :64] = bf16(h0)
+// h0 = relu(f W_in + b_in), X0[:, :64] = bf16(h0). Memory-bound by its stores: 16
+// lanes per node, four features each, walk the nodes with their weights in
+// registers (a thread per feature loaded four weights and four node values for
+// each word it stored: 51 -> 24 us at 262,144 nodes; 15 us of traffic).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_encode(const float *fd, const float *fs, const T *r, const float *rms, const float *P, float *H, bf16 *X, long long n)
 {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n * kHid) return;
-    const long long i = idx / kHid;
-    const int j = (int)(idx % kHid);
-    const float f2 = (float)r[i] * rms[1];
-    const float z = fd[i] * P[kOffWin + j] + fs[i] * P[kOffWin + kHid + j] + f2 * P[kOffWin + 2 * kHid + j] +
-                    P[kOffBin + j];
-    const float h = relu(z);
-    H[idx] = h;
-    X[i * 128 + j] = __float2bfloat16_rn(h);
+    const int j = (threadIdx.x & 15) * 4, sub = threadIdx.x >> 4;
+    const float4 w0 = *reinterpret_cast<const float4 *>(P + kOffWin + j);
+    const float4 w1 = *reinterpret_cast<const float4 *>(P + kOffWin + kHid + j);
+    const float4 w2 = *reinterpret_cast<const float4 *>(P + kOffWin + 2 * kHid + j);
+    const float4 b = *reinterpret_cast<const float4 *>(P + kOffBin + j);
+    const float ri = rms[1];
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * 16 + sub; i < n; i += (long long)gridDim.x * 16) {
+        const float f0 = fd[i], f1 = fs[i], f2 = (float)r[i] * ri;
+        float4 h;
+        h.x = relu(f0 * w0.x + f1 * w1.x + f2 * w2.x + b.x);
+        h.y = relu(f0 * w0.y + f1 * w1.y + f2 * w2.y + b.y);
+        h.z = relu(f0 * w0.z + f1 * w1.z + f2 * w2.z + b.z);
+        h.w = relu(f0 * w0.w + f1 * w1.w + f2 * w2.w + b.w);
+        *reinterpret_cast<float4 *>(H + i * kHid + j) = h;
+        st_bf16x4(X + i * 128 + j, h.x, h.y, h.z, h.w);
+    }
 }
 
 // m = W h, 8 lanes per row (4 rows per warp), lane k of a row holding
@@ -228,37 +238,46 @@ k_relu_back(const float *dH, const bf16 *Z, bf16 *dZ, float *gbeta, long long n)
 }
 
 // Encoder backward: dz = dH0 (.) [z0 > 0] (z0 recomputed); grad W_in += f dz, grad b_in += dz.
+// 16 nodes x 16 groups of four features per pass, as k_relu_back: 54 -> 26 us at
+// 262,144 nodes, with a feature per thread before (11 us of traffic).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_encode_back(const float *fd, const float *fs, const T *r, const float *rms, const float *P, const float *dH, float *G,
               long long n)
 {
-    const int j = threadIdx.x & 63, sub = threadIdx.x >> 6;
-    float s0 = 0, s1 = 0, s2 = 0, sb = 0;
-    const float w0 = P[kOffWin + j], w1 = P[kOffWin + kHid + j], w2 = P[kOffWin + 2 * kHid + j], b = P[kOffBin + j];
-    for (long long i = (long long)blockIdx.x * 4 + sub; i < n; i += (long long)gridDim.x * 4) {
-        const float f2 = (float)r[i] * rms[1];
-        const float z = fd[i] * w0 + fs[i] * w1 + f2 * w2 + b;
-        const float g = z > 0.f ? dH[i * 64 + j] : 0.f;
-        s0 += g * fd[i];
-        s1 += g * fs[i];
-        s2 += g * f2;
-        sb += g;
+    const int j = (threadIdx.x & 15) * 4, sub = threadIdx.x >> 4;
+    float w[4][4], s[4][4] = {};  // [W_in rows, b_in][feature]
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) w[q][k] = P[(q < 3 ? kOffWin + q * kHid : kOffBin) + j + k];
     }
-    __shared__ float sh[4][4][64];
-    sh[0][sub][j] = s0;
-    sh[1][sub][j] = s1;
-    sh[2][sub][j] = s2;
-    sh[3][sub][j] = sb;
+    const float ri = rms[1];
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * 16 + sub; i < n; i += (long long)gridDim.x * 16) {
+        const float f0 = fd[i], f1 = fs[i], f2 = (float)r[i] * ri;
+        const float4 d4 = __ldg(reinterpret_cast<const float4 *>(dH + i * kHid + j));
+        const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float z = f0 * w[0][k] + f1 * w[1][k] + f2 * w[2][k] + w[3][k];
+            const float g = z > 0.f ? d[k] : 0.f;
+            s[0][k] += g * f0;
+            s[1][k] += g * f1;
+            s[2][k] += g * f2;
+            s[3][k] += g;
+        }
+    }
+    __shared__ __align__(16) float sh[4][16][kHid];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        *reinterpret_cast<float4 *>(&sh[q][sub][j]) = make_float4(s[q][0], s[q][1], s[q][2], s[q][3]);
     __syncthreads();
-    if (threadIdx.x < 64) {
-        float a[4];
-        for (int q = 0; q < 4; q++) a[q] = sh[q][0][j] + sh[q][1][j] + sh[q][2][j] + sh[q][3][j];
-        atomicAdd(G + kOffWin + j, a[0]);
-        atomicAdd(G + kOffWin + kHid + j, a[1]);
-        atomicAdd(G + kOffWin + 2 * kHid + j, a[2]);
-        atomicAdd(G + kOffBin + j, a[3]);
-    }
+    const int q = threadIdx.x >> 6, c = threadIdx.x & 63;
+    float a = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; k++) a += sh[q][k][c];
+    atomicAdd(G + (q < 3 ? kOffWin + q * kHid : kOffBin) + c, a);
 }
 
 // Adam (decoupled moments, bias-corrected), then the BF16 weight copies:
@@ -300,15 +319,24 @@ __global__ void __launch_bounds__(kThreads) k_weights_bf16(const float *P, bf16 
     WTb[(long long)l * 128 * 64 + j * 128 + i] = v;  // Theta_l^T[j][i]
 }
 
-// c_i = h_i . w_out + b_out, warp per node
+// c_i = h_i . w_out + b_out, a warp for four nodes: their loads and their
+// reductions overlap (26 -> 13 us at 262,144 nodes, 10 us of traffic)
 __global__ void __launch_bounds__(kThreads) k_decode_c(const float *H, const float *P, float *c, long long n)
 {
-    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    constexpr int U = 4;
+    const long long i = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * U;
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
-    const float2 h = *reinterpret_cast<const float2 *>(H + i * 64 + 2 * lane);
-    const float v = warp_sum(h.x * P[kOffWout + 2 * lane] + h.y * P[kOffWout + 2 * lane + 1]);
-    if (lane == 0) c[i] = v + P[kOffBout];
+    float2 h[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        h[u] = i + u < n ? *reinterpret_cast<const float2 *>(H + (i + u) * 64 + 2 * lane) : make_float2(0.f, 0.f);
+    const float w0 = P[kOffWout + 2 * lane], w1 = P[kOffWout + 2 * lane + 1], b = P[kOffBout];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const float v = warp_sum(h[u].x * w0 + h[u].y * w1);
+        if (lane == 0 && i + u < n) c[i + u] = v + b;
+    }
 }
 
 // Least-squares step of the correction: alpha = (q . y) / (y . y) with
@@ -410,37 +438,39 @@ k_spmv_grad(const int *rp, const int *ci, const float *bv, const float *e, float
     }
 }
 
-// Decoder backward: dH4 = dc w_out; grad w_out += dc h; grad b_out += dc (warp per node)
+// Decoder backward: dH4 = dc w_out; grad w_out += dc h; grad b_out += dc.
+// 16 nodes x 16 groups of four features per pass, as k_relu_back (a warp per
+// node had too few loads in flight: 33 -> 22 us at 262,144 nodes, 20 us of traffic).
 __global__ void __launch_bounds__(kThreads)
 k_decode_back(const float *H, const float *P, const float *dc, float *dH, float *G, long long n)
 {
-    __shared__ float gw[kThreads / 32][kHid];
-    __shared__ float gb[kThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const float w0 = P[kOffWout + 2 * lane], w1 = P[kOffWout + 2 * lane + 1];
-    float g0 = 0.f, g1 = 0.f, gbs = 0.f;
-    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const float2 h = *reinterpret_cast<const float2 *>(H + i * 64 + 2 * lane);
-        const float g = dc[i];
-        *reinterpret_cast<float2 *>(dH + i * 64 + 2 * lane) = make_float2(g * w0, g * w1);
-        g0 += g * h.x;
-        g1 += g * h.y;
-        gbs += g;
+    const int j = (threadIdx.x & 15) * 4, sub = threadIdx.x >> 4;
+    // w_out and its gradient start at an offset of the parameters that is a multiple of four
+    static_assert(kOffWout % 4 == 0, "16-byte loads of w_out");
+    const float4 w = *reinterpret_cast<const float4 *>(P + kOffWout + j);
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    float gb = 0.f;
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * 16 + sub; i < n; i += (long long)gridDim.x * 16) {
+        const float4 h = __ldg(reinterpret_cast<const float4 *>(H + i * 64 + j));
+        const float v = __ldg(dc + i);
+        *reinterpret_cast<float4 *>(dH + i * 64 + j) = make_float4(v * w.x, v * w.y, v * w.z, v * w.w);
+        g.x += v * h.x;
+        g.y += v * h.y;
+        g.z += v * h.z;
+        g.w += v * h.w;
+        gb += v;
     }
-    gw[wid][2 * lane] = g0;
-    gw[wid][2 * lane + 1] = g1;
-    if (lane == 0) gb[wid] = gbs;
+    __shared__ __align__(16) float sh[16][kHid];
+    __shared__ float sb[16];
+    *reinterpret_cast<float4 *>(&sh[sub][j]) = g;
+    if (j == 0) sb[sub] = gb;
     __syncthreads();
-    if (threadIdx.x < kHid) {
-        float s = 0;
-        for (int w = 0; w < kThreads / 32; w++) s += gw[w][threadIdx.x];
-        atomicAdd(G + kOffWout + threadIdx.x, s);
-    }
-    if (threadIdx.x == 0) {
-        float s = 0;
-        for (int w = 0; w < kThreads / 32; w++) s += gb[w];
-        atomicAdd(G + kOffBout, s);
+    if (threadIdx.x <= kHid) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; k++) t += threadIdx.x < kHid ? sh[k][threadIdx.x] : sb[k];
+        atomicAdd(G + (threadIdx.x < kHid ? kOffWout + threadIdx.x : kOffBout), t);
     }
 }
 
@@ -604,7 +634,7 @@ struct Mpnn {
     {
         const int rg = std::min(ceil_div(n, kThreads), sm_count() * 4);
         k_rms<T><<<rg, kThreads, 0, s>>>(r, n, red.p, ticket.p, rms.p);
-        k_encode<T><<<ceil_div(n * kHid, kThreads), kThreads, 0, s>>>(fd.p, fs.p, r, rms.p, P.p, H[0].p, X[0].p, n);
+        k_encode<T><<<std::min(ceil_div(n, 16), sm_count() * 8), kThreads, 0, s>>>(fd.p, fs.p, r, rms.p, P.p, H[0].p, X[0].p, n);
         const int tiles = ceil_div(n, 128);
         for (int l = 0; l < kLayers; l++) {
             k_aggregate<<<ceil_div(n * 8, kThreads), kThreads, 0, s>>>(wr.p, wc.p, wv.p, X[l].p, n);
@@ -665,7 +695,7 @@ struct Mpnn {
         SENK_CUDA(cudaMemsetAsync(acc.p, 0, acc.bytes(), s));
         forward<T>(r, s, true);
         const int rg = std::min(ceil_div(n, kThreads), sm_count() * 4);
-        k_decode_c<<<ceil_div(n * 32, kThreads), kThreads, 0, s>>>(H[kLayers].p, P.p, cbuf.p, n);
+        k_decode_c<<<ceil_div(ceil_div(n, 4) * 32LL, kThreads), kThreads, 0, s>>>(H[kLayers].p, P.p, cbuf.p, n);
         if (loss_mode == 0) {
             k_target<T><<<rg, kThreads, 0, s>>>(e, ilu, rms.p, d, t.p, n, red.p, ticket.p, acc.p);
             k_loss_error<<<rg, kThreads, 0, s>>>(cbuf.p, t.p, dcb.p, acc.p, n);
@@ -674,7 +704,7 @@ struct Mpnn {
             k_spmv_loss<<<rg, kThreads, 0, s>>>(ar.p, ac.p, av.p, cbuf.p, ebuf.p, n, 1.f / d, t.p, acc.p);
             k_spmv_grad<<<rg, kThreads, 0, s>>>(atr.p, atc.p, atv.p, ebuf.p, dcb.p, n, 1.f / d, acc.p);
         }
-        k_decode_back<<<sm_count() * 4, kThreads, 0, s>>>(H[kLayers].p, P.p, dcb.p, dH.p, G.p, n);
+        k_decode_back<<<sm_count() * 8, kThreads, 0, s>>>(H[kLayers].p, P.p, dcb.p, dH.p, G.p, n);
         float *dh = dH.p, *dh2 = dH2.p;
         const int tiles = ceil_div(n, 128);
         for (int l = kLayers - 1; l >= 0; l--) {
