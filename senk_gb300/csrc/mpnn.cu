@@ -32,6 +32,7 @@ constexpr int kSmemFwd = tc_gemm_smem(128, 64);  // 48 KB of operand tiles
 constexpr int kSmemDx = tc_gemm_smem(64, 128);   // 66 KB: the 128 x 132 FP32 result tile
 constexpr int kSmemTn = TnLayout<64>::kBytes;    // 100 KB of pipeline stages: 2 CTAs x 64 columns
 
+constexpr int kAggCtas = 8;  // per SM, of k_aggregate_back<true>
 constexpr int kHid = 64;
 constexpr int kLayers = 4;
 constexpr int kIn = 3;
@@ -129,42 +130,82 @@ k_aggregate(const int *__restrict__ rptr, const int *__restrict__ cind, const fl
 }
 
 // dH += W^T dM (fp32), 8 lanes per row of W^T (4 rows per warp), lane k of a
-// row holding features 8k..8k+7 (two 16-byte loads per entry).
+// row holding features 8k..8k+7 (two 16-byte loads per entry). With RELU, while
+// the new dH is in registers, also what the layer below starts with (Z, dZ, gbeta
+// its own): dZ = bf16(dH (.) [z > 0]), gbeta += column sums of the FP32 product;
+// the CTAs then walk the rows, so that few of them add their sums. A pass of its
+// own for that took 22 us at 262,144 rows, beside 57 here: loss and gradient 1390
+// -> 1333 us (1344 with 4 CTAs to an SM, 1342 with 16, 1356 with 32).
+template <bool RELU>
 __global__ void __launch_bounds__(kThreads)
 k_aggregate_back(const int *__restrict__ rptr, const int *__restrict__ cind, const float *__restrict__ w,
-                 const float *__restrict__ dM, float *__restrict__ dH, long long n)
+                 const float *__restrict__ dM, float *__restrict__ dH, const bf16 *__restrict__ Z,
+                 bf16 *__restrict__ dZ, float *gbeta, long long n)
 {
-    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int sub = threadIdx.x & 7;
-    if (row >= n) return;
-    float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-    const int p1 = rptr[row + 1];
+    float s[8] = {};
+    for (long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; row < n;
+         row += ((long long)gridDim.x * blockDim.x) >> 3) {
+        float4 *o = reinterpret_cast<float4 *>(dH + row * 64 + 8 * sub);
+        float4 v0 = o[0], v1 = o[1];
+        uint4 zz = make_uint4(0, 0, 0, 0);
+        if (RELU) zz = *reinterpret_cast<const uint4 *>(Z + row * 64 + 8 * sub);
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+        const int p1 = rptr[row + 1];
 #pragma unroll 4
-    for (int p = rptr[row]; p < p1; p++) {
-        const float wv = w[p];
-        const float4 *d = reinterpret_cast<const float4 *>(dM + (long long)cind[p] * 64 + 8 * sub);
-        const float4 d0 = d[0], d1 = d[1];
-        a0.x += wv * d0.x;
-        a0.y += wv * d0.y;
-        a0.z += wv * d0.z;
-        a0.w += wv * d0.w;
-        a1.x += wv * d1.x;
-        a1.y += wv * d1.y;
-        a1.z += wv * d1.z;
-        a1.w += wv * d1.w;
+        for (int p = rptr[row]; p < p1; p++) {
+            const float wv = w[p];
+            const float4 *d = reinterpret_cast<const float4 *>(dM + (long long)cind[p] * 64 + 8 * sub);
+            const float4 d0 = d[0], d1 = d[1];
+            a0.x += wv * d0.x;
+            a0.y += wv * d0.y;
+            a0.z += wv * d0.z;
+            a0.w += wv * d0.w;
+            a1.x += wv * d1.x;
+            a1.y += wv * d1.y;
+            a1.z += wv * d1.z;
+            a1.w += wv * d1.w;
+        }
+        v0.x += a0.x;
+        v0.y += a0.y;
+        v0.z += a0.z;
+        v0.w += a0.w;
+        v1.x += a1.x;
+        v1.y += a1.y;
+        v1.z += a1.z;
+        v1.w += a1.w;
+        o[0] = v0;
+        o[1] = v1;
+        if (RELU) {
+            const __nv_bfloat162 *z = reinterpret_cast<const __nv_bfloat162 *>(&zz);
+            const float d[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            uint4 out;
+            uint32_t *ow = reinterpret_cast<uint32_t *>(&out);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float gx = __bfloat162float(z[k].x) > 0.f ? d[2 * k] : 0.f;
+                const float gy = __bfloat162float(z[k].y) > 0.f ? d[2 * k + 1] : 0.f;
+                const __nv_bfloat162 v = __floats2bfloat162_rn(gx, gy);
+                ow[k] = *reinterpret_cast<const uint32_t *>(&v);
+                s[2 * k] += gx;
+                s[2 * k + 1] += gy;
+            }
+            *reinterpret_cast<uint4 *>(dZ + row * 64 + 8 * sub) = out;
+        }
     }
-    float4 *o = reinterpret_cast<float4 *>(dH + row * 64 + 8 * sub);
-    float4 v0 = o[0], v1 = o[1];
-    v0.x += a0.x;
-    v0.y += a0.y;
-    v0.z += a0.z;
-    v0.w += a0.w;
-    v1.x += a1.x;
-    v1.y += a1.y;
-    v1.z += a1.z;
-    v1.w += a1.w;
-    o[0] = v0;
-    o[1] = v1;
+    if (RELU) {
+        __shared__ __align__(16) float sh[kThreads / 8][kHid];
+        float4 *d = reinterpret_cast<float4 *>(&sh[threadIdx.x >> 3][8 * sub]);
+        d[0] = make_float4(s[0], s[1], s[2], s[3]);
+        d[1] = make_float4(s[4], s[5], s[6], s[7]);
+        __syncthreads();
+        if (threadIdx.x < kHid) {
+            float t = 0.f;
+#pragma unroll
+            for (int k = 0; k < kThreads / 8; k++) t += sh[k][threadIdx.x];
+            atomicAdd(gbeta + threadIdx.x, t);
+        }
+    }
 }
 
 // Inference epilogue: out_i = ilu_i + (rms / d) * (h_i . w_out + b_out); warp per node.
@@ -707,9 +748,10 @@ struct Mpnn {
         k_decode_back<<<sm_count() * 8, kThreads, 0, s>>>(H[kLayers].p, P.p, dcb.p, dH.p, G.p, n);
         float *dh = dH.p, *dh2 = dH2.p;
         const int tiles = ceil_div(n, 128);
+        auto gbeta = [&](int l) { return G.p + kOffLayer + l * kLayerSize + 2 * kHid * kHid; };
+        k_relu_back<<<sm_count() * 8, kThreads, 0, s>>>(dh, Z[kLayers - 1].p, dZ.p, gbeta(kLayers - 1), n);
         for (int l = kLayers - 1; l >= 0; l--) {
             float *gl = G.p + kOffLayer + l * kLayerSize;
-            k_relu_back<<<sm_count() * 8, kThreads, 0, s>>>(dh, Z[l].p, dZ.p, gl + 2 * kHid * kHid, n);
             k_tc_gemm_tn<64><<<sm_count() * 2, 128, kSmemTn, s>>>(X[l].p, 128, dZ.p, (int)n, gl, status.p);
             TcArgs a;
             a.hin = dh;
@@ -717,7 +759,12 @@ struct Mpnn {
             a.dm = dM.p;
             k_tc_gemm<64, 128, kTcDx><<<tiles, 128, kSmemDx, s>>>(
                 dZ.p, 64, Wb.p + (size_t)l * 128 * 64, (int)n, a, status.p);
-            k_aggregate_back<<<ceil_div(n * 8, kThreads), kThreads, 0, s>>>(tr.p, tcol.p, tv.p, dM.p, dh2, n);
+            if (l > 0)
+                k_aggregate_back<true><<<std::min(ceil_div(n * 8, kThreads), sm_count() * kAggCtas), kThreads, 0, s>>>(
+                    tr.p, tcol.p, tv.p, dM.p, dh2, Z[l - 1].p, dZ.p, gbeta(l - 1), n);
+            else
+                k_aggregate_back<false><<<ceil_div(n * 8, kThreads), kThreads, 0, s>>>(
+                    tr.p, tcol.p, tv.p, dM.p, dh2, nullptr, nullptr, nullptr, n);
             std::swap(dh, dh2);
         }
         k_encode_back<T><<<sm_count() * 8, kThreads, 0, s>>>(fd.p, fs.p, r, rms.p, P.p, dh, G.p, n);
