@@ -146,6 +146,7 @@ struct BlGroup {
 };
 
 constexpr int kBlMaxSteps = 16;
+constexpr int kBlMaxGroups = 14;  // to an SM, mean of the colours, FP64 (IlubPlan::build_slices)
 
 // Byte offsets of a group's staged part: widths (external, in-chain) of each
 // step, the external block columns, the in-chain columns (scalar, from the
@@ -228,20 +229,20 @@ k_ilub_fill(const BlGroup *__restrict__ groups, const uint16_t *__restrict__ wid
                 live ? bval[(size_t)(brptr[br] + c / BNW) * BS + (c % BNW) * BNL + r] : T(0);
 }
 
-// t -= v[k][l] * gy[k][l] over the last n of 4 slots, in order (n the same in
+// t -= v[k][l] * gy[k][l] over the last n of B slots, in order (n the same in
 // the whole warp); the entry is a jump, see sub_last.
-template <int BNW, typename T>
-__device__ __forceinline__ void sub_slots(T &t, const T (&v)[4][BNW], const T *gy, int stride, int n)
+template <int BNW, int B, typename T>
+__device__ __forceinline__ void sub_slots(T &t, const T (&v)[B][BNW], const T *gy, int stride, int n)
 {
     auto slot = [&](int k) {
 #pragma unroll
         for (int l = 0; l < BNW; l++) t -= v[k][l] * gy[k * stride + l];
     };
     switch (n) {
-    case 4: slot(0);
-    case 3: slot(1);
-    case 2: slot(2);
-    case 1: slot(3);
+    case 4: if constexpr (B >= 4) slot(B - 4);
+    case 3: if constexpr (B >= 3) slot(B - 3);
+    case 2: slot(B - 2);
+    case 1: slot(B - 1);
     default: break;
     }
 }
@@ -249,21 +250,26 @@ __device__ __forceinline__ void sub_slots(T &t, const T (&v)[4][BNW], const T *g
 // One colour per launch, one CTA per group: the block rows of earlier colours
 // that the group's external slots name are gathered into shared memory, warp q
 // subtracts the external slots of step q (their values read straight into
-// registers, four slots ahead), and one warp runs the in-chain part step by
+// registers, a batch of slots ahead), and one warp runs the in-chain part step by
 // step, as k_ilub_sweep does. The staged part (TMA), the first external values
 // and, with early_x, x and the gate are read before the wait on the previous
 // kernel. Same operations in the same order as k_ilub_sweep, which walked a
 // chain's block rows one after another with a dependent gather per four blocks.
 // Block-3x3 system, 48^3 nodes (8 colours), one application: FP64 0.524 ->
-// 0.177 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
+// 0.149 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
 // row's up to 69 FP64 subtractions at 65 cycles, then four in-chain steps) and
-// by the FP64 unit (50 us of the 177).
+// by the FP64 unit (50 us of the 149). FP64 takes two slots ahead in 64
+// registers: more CTAs on an SM hide those steps better than four slots in 80
+// do (48^3 0.177 ms, 80^3 0.446 against 0.430, 96^3 0.778 against 0.720; 64^3
+// 0.238 against 0.246).
+template <typename T> constexpr int bl_batch = sizeof(T) == 8 ? 2 : 4;
+template <typename T> constexpr int bl_min_blocks = sizeof(T) == 8 ? 4 : 0;  // 0: not stated
 template <typename T, int BNL, int BNW, bool UPPER>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, bl_min_blocks<T>)
 k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const T *__restrict__ ext,
               const uint4 *__restrict__ blob, const T *x, T *y, const int *gate, int *status, int early_x)
 {
-    constexpr int RPW = 32 / BNL, B = 4;
+    constexpr int RPW = 32 / BNL, B = bl_batch<T>;
     extern __shared__ __align__(128) unsigned char bls[];
     __shared__ __align__(8) unsigned long long bar;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
@@ -350,7 +356,7 @@ k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const 
             const T *gk = gy + ((s0 + k1 - B) * RPW + at) * BNW;  // used from the first slot in use on
             const int next = k1 + B;
             if (k1 < width) load(s0, next);
-            sub_slots<BNW>(t, cur, gk, RPW * BNW, m);
+            sub_slots<BNW, B>(t, cur, gk, RPW * BNW, m);
             k1 = k1 < width ? next : 0;
         }
         if (g < RPW && row < nrows) ysh[row] = t;
@@ -568,6 +574,13 @@ bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, c
         if ((int)gd.size() > before) F.launches.push_back({before, (int)gd.size(), 0});
     }
     const int ng = (int)gd.size();
+    // FP64 colours of many groups to an SM: k_ilub_sweep, which then has enough
+    // chains to hide its latencies, reads y and the factor once and no padding.
+    // Block-3x3 system: 10.5 groups to an SM and colour (80^3 nodes) 0.430 ms
+    // against its 0.623, GCR(20) 17.4 against 20.9; 18.2 (96^3) 0.720 against
+    // 0.752, but GCR(20), its vectors and factors cold, 34.6 against 31.2 (with four
+    // slots ahead, 0.778). FP32 is faster in slices there too (0.317 against 0.472).
+    if (sizeof(T) == 8 && ng > (long long)kBlMaxGroups * sm_count() * (long long)F.launches.size()) return false;
     std::vector<uint16_t> widths((size_t)ng * 2 * per, 0);
     bool fits = true;
 #pragma omp parallel for schedule(static) reduction(&& : fits)

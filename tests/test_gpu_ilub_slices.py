@@ -63,3 +63,37 @@ def test_system_precond(port, dtype, tol):
     wl = port.ilub_sweep(bl, x.astype(np.float64), False, 3, 3, sc, nc, 12)
     want = port.ilub_sweep(bu, wl, True, 3, 3, sc, nc, 12)
     assert np.max(np.abs(got - want)) <= tol * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("rows", [67968, 68001, 68352])  # the last: more groups to an SM than the slices take
+def test_many_groups(port, rows):
+    """Two colours of single 2x2 block rows, red rows first, each black row
+    coupled with two red ones, around the group count from which k_ilub_sweep runs."""
+    import torch
+    rng = np.random.default_rng(rows)
+    red = (rows + 1) // 2
+    black = np.arange(rows - red)
+    pair = np.stack([black, np.minimum(black + 1, red - 1)], 1).astype(np.int32)
+    lp = np.zeros(rows + 1, np.int32)
+    lp[red + 1:] = 2 * np.arange(1, rows - red + 1)
+    bl = (rng.uniform(-.3, .3, 8 * len(black)), pair.reshape(-1), lp)
+    up, uc, uv = np.zeros(rows + 1, np.int32), [], []
+    cnt = np.where(np.arange(rows) < red, 2, 1)
+    cnt[:red][np.arange(red) >= rows - red] = 1    # a red row without a black partner
+    up[1:] = np.cumsum(cnt)
+    uc = np.zeros(up[-1], np.int32)
+    uc[up[:-1]] = np.arange(rows)
+    two = np.flatnonzero(cnt == 2)
+    uc[up[two] + 1] = red + two
+    uv = rng.uniform(-.3, .3, (up[-1], 4))
+    uv[up[:-1]] = np.array([1.0, 0.0, 0.2, 0.5])   # inverted diagonal square, column-major
+    bu = (uv.reshape(-1), uc, up)
+    sc = np.array([0, red, rows], np.int32)
+    plan = IlubPlan(bl, bu, 2 * rows, 2, 2, sc, 2, 2)
+    L.check("plan", plan.code)
+    x = rng.uniform(-1, 1, 2 * rows)
+    y = torch.from_numpy(x).cuda()
+    L.check("apply", L.lib().senk_ilu_plan_apply(plan.h, y.data_ptr(), y.data_ptr(), None))
+    L.check("status", L.lib().senk_ilu_plan_status(plan.h, None))
+    want = port.ilub_sweep(bu, port.ilub_sweep(bl, x, False, 2, 2, sc, 2, 2), True, 2, 2, sc, 2, 2)
+    assert np.max(np.abs(y.cpu().numpy() - want)) <= 1e-12 * np.max(np.abs(want))
