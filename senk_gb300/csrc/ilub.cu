@@ -256,9 +256,9 @@ __device__ __forceinline__ void sub_slots(T &t, const T (&v)[B][BNW], const T *g
 // kernel. Same operations in the same order as k_ilub_sweep, which walked a
 // chain's block rows one after another with a dependent gather per four blocks.
 // Block-3x3 system, 48^3 nodes (8 colours), one application: FP64 0.524 ->
-// 0.149 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
+// 0.151 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
 // row's up to 69 FP64 subtractions at 65 cycles, then four in-chain steps) and
-// by the FP64 unit (50 us of the 149). FP64 takes two slots ahead in 64
+// by the FP64 unit (50 us of the 151). FP64 takes two slots ahead in 64
 // registers: more CTAs on an SM hide those steps better than four slots in 80
 // do (48^3 0.177 ms, 80^3 0.446 against 0.430, 96^3 0.778 against 0.720; 64^3
 // 0.238 against 0.246).
