@@ -146,6 +146,7 @@ struct BlGroup {
 };
 
 constexpr int kBlMaxSteps = 16;
+constexpr size_t kBlMaxSmem = 160 * 1024;  // shared memory of a group; the kernels' limit for every plan
 constexpr int kBlMaxGroups = 14;  // to an SM, mean of the colours, FP64 (IlubPlan::build_slices)
 
 // Byte offsets of a group's staged part: widths (external, in-chain) of each
@@ -621,15 +622,13 @@ bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, c
         ext += we;
         blob += parts.end / 16;
         smem[g] = parts.end + ((size_t)rpw * kBlMaxSteps * bnl + (size_t)we * rpw * bnw) * sizeof(T);
-        if (smem[g] > 160 * 1024 || ext >= (1 << 30) || blob >= (1 << 30)) return false;
+        if (smem[g] > kBlMaxSmem || ext >= (1 << 30) || blob >= (1 << 30)) return false;
     }
     gd.push_back({0, 0, (int)ext, (int)blob});
-    size_t most = 48 * 1024;
     for (size_t k = 0; k < F.launches.size(); k++) {
         auto &L = F.launches[k];
         L.early_x = k > 0;
         for (int g = L.g0; g < L.g1; g++) L.smem = std::max(L.smem, smem[g]);
-        most = std::max(most, L.smem);
     }
     F.groups.alloc(gd.size());
     F.groups.upload((const int4 *)gd.data(), gd.size(), s);
@@ -644,12 +643,12 @@ bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, c
             k_ilub_fill<T, R, C, true><<<ng, 32 * per, 0, s>>>(dg, dw.p, per, nbr, uval.p, ucind.p, urptr.p, F.ext.p, \
                                                                F.blob.p);                                        \
             SENK_CUDA(cudaFuncSetAttribute(k_ilub_slices<T, R, C, true>,                                         \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));             \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlMaxSmem));       \
         } else {                                                                                                 \
             k_ilub_fill<T, R, C, false><<<ng, 32 * per, 0, s>>>(dg, dw.p, per, nbr, lval.p, lcind.p, lrptr.p,    \
                                                                 F.ext.p, F.blob.p);                              \
             SENK_CUDA(cudaFuncSetAttribute(k_ilub_slices<T, R, C, false>,                                        \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));             \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlMaxSmem));       \
         }                                                                                                        \
     } else
     SENK_ILUB_SHAPES(X)

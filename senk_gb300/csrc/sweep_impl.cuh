@@ -197,6 +197,15 @@ constexpr size_t kMaxStagedBytes = 160 * 1024;
 // Largest dynamic shared memory of one dataflow CTA.
 constexpr size_t kMaxWfSmem = 200 * 1024;
 
+// A kernel's limit on dynamic shared memory belongs to the function, so every
+// plan sets it to the most that any plan may launch the kernel with, never to
+// its own need: a plan with smaller groups would lower it for the plans before.
+template <typename... A>
+void allow_dynamic(void (*kern)(A...), size_t bytes)
+{
+    SENK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // Largest vector the single-CTA sweeps of small systems keep in shared memory,
 // and the most dynamic shared memory of that kernel (vector + two staging
 // buffers).
@@ -350,8 +359,8 @@ bool build_factor_lv(SweepFactor<VT> &F, int N, const VT *val, const int *cind, 
     drptr.upload(rptr, (size_t)N + 1, s);
     djobs.upload(jobs.data(), jobs.size(), s);
     constexpr int smem = (int)sizeof(LvBuildShared);
-    SENK_CUDA(cudaFuncSetAttribute(k_lv_build<VT, UPPER, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    SENK_CUDA(cudaFuncSetAttribute(k_lv_build<VT, UPPER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    allow_dynamic(k_lv_build<VT, UPPER, false>, smem);
+    allow_dynamic(k_lv_build<VT, UPPER, true>, smem);
     k_lv_build<VT, UPPER, false><<<ng, kLvMaxRows, smem, s>>>(djobs.p, dval.p, dcind.p, drptr.p, N, bs, nullptr,
                                                               nullptr, dsize.p);
     SENK_LAUNCH_CHECK();
@@ -483,8 +492,7 @@ void launch_colour(const SweepFactor<VT> &F, int *status, int c, const XT *x, XT
 template <typename VT, typename XT, int BS, bool UPPER, bool MAPPED>
 void allow_smem()
 {
-    SENK_CUDA(cudaFuncSetAttribute(k_sweep<VT, XT, BS, UPPER, MAPPED, true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStagedBytes));
+    allow_dynamic(k_sweep<VT, XT, BS, UPPER, MAPPED, true>, kMaxStagedBytes);
 }
 
 template <typename VT, typename XT, int BS, bool UPPER>
@@ -584,15 +592,10 @@ void launch_cc(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
 template <typename VT, int BS, bool UPPER>
 void shape_cc(SweepFactor<VT> &F)
 {
-    size_t most = 0;
-    for (const auto &L : F.launches) most = std::max(most, L.smem);
-    const int lim = (int)std::max<size_t>(most, 48 * 1024);
     if (F.rowlane) {
-        SENK_CUDA(cudaFuncSetAttribute(k_sweep_rl<VT, VT, BS, UPPER, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       lim));
+        allow_dynamic(k_sweep_rl<VT, VT, BS, UPPER, 1>, kMaxWfSmem);
         if constexpr (BS >= 2) {
-            SENK_CUDA(cudaFuncSetAttribute(k_sweep_rl<VT, VT, BS, UPPER, 2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+            allow_dynamic(k_sweep_rl<VT, VT, BS, UPPER, 2>, kMaxWfSmem);
             for (auto &L : F.launches) {
                 if (L.coop) continue;
                 if (F.force_wide) {
@@ -609,10 +612,9 @@ void shape_cc(SweepFactor<VT> &F)
         }
         return;
     }
-    SENK_CUDA(cudaFuncSetAttribute(k_sweep_cc<VT, VT, BS, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    allow_dynamic(k_sweep_cc<VT, VT, BS, UPPER>, kMaxWfSmem);
     if constexpr (BS >= 4) {
-        SENK_CUDA(cudaFuncSetAttribute(k_sweep_cc2<VT, VT, BS, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       lim));
+        allow_dynamic(k_sweep_cc2<VT, VT, BS, UPPER>, kMaxWfSmem);
         for (auto &L : F.launches) {
             if (L.coop) continue;
             if (F.force_wide) {
@@ -651,17 +653,15 @@ void launch_lv(const SweepFactor<VT> &F, int *status, const VT *x, VT *y, cudaSt
     }
 }
 
-// Shared memory limits of k_sweep_lv, and which colours take half the threads
+// Shared memory limit of k_sweep_lv, and which colours take half the threads
 // (two slices per warp): those with more groups than one wave of full-width
 // CTAs holds.
 template <typename VT, bool UPPER>
 void shape_lv(SweepFactor<VT> &F)
 {
     auto full = k_sweep_lv<VT, UPPER, kLvMaxRows>, half = k_sweep_lv<VT, UPPER, kLvMaxRows / 2>;
-    size_t most = 48 * 1024;
-    for (const auto &L : F.launches) most = std::max(most, L.smem);
-    SENK_CUDA(cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    SENK_CUDA(cudaFuncSetAttribute(half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    allow_dynamic(full, kMaxStagedBytes);
+    allow_dynamic(half, kMaxStagedBytes);
     for (auto &L : F.launches) {
         if (L.rows < 64) continue;
         int one = 0, two = 0;
@@ -690,8 +690,7 @@ void shape_cp(SweepFactor<VT> &F)
     buf = (buf + 127) / 128 * 128;
     if (2 * buf > kMaxWfSmem) return;
     auto kern = k_sweep_cp<VT, VT, BS, UPPER>;
-    SENK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)std::max<size_t>(2 * buf, 48 * 1024)));
+    allow_dynamic(kern, kMaxWfSmem);
     int per_sm = 0;
     SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BS * 32, 2 * buf));
     if (per_sm < 1) return;
@@ -740,7 +739,7 @@ void shape_wf(SweepFactor<VT> &F)
     warps = std::min(warps, std::max(1, F.ngroups));
     F.wf_warps = warps;
     F.wf_smem = per_warp * warps;
-    SENK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F.wf_smem));
+    allow_dynamic(kern, kMaxWfSmem);
     int per_sm = 0;
     SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, F.wf_smem));
     SENK_REQUIRE(per_sm >= 1, "the dataflow sweep does not fit an SM");
@@ -931,11 +930,10 @@ void IluPlan<VT>::build_small(int N, const VT *lval, const int *lcind, const int
     // that the rounds over a level's rows weigh more than the hand-over
     small_sets = most <= 240 && small_nbuf > 4 ? 4 : most <= 480 ? 2 : 1;
     small_threads = small_sets > 1 ? small_sets * most : std::min(992, most);
-    const size_t smem = small_smem_bytes((size_t)N, sizeof(VT), steps, small_buf, small_nbuf);
     small_fast = small_sets > 1;
     for (int i = 0; i < N; i++)
         small_fast = small_fast && lrptr[i + 1] - lrptr[i] <= 3 && urptr[i + 1] - urptr[i] <= 4;
-    SENK_CUDA(cudaFuncSetAttribute(small_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dynamic(small_kernel(), kSmallSmem);
     small = true;
 }
 
