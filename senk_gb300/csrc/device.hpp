@@ -290,7 +290,7 @@ struct IlubPlan {
     struct Slices {
         struct Launch {
             int g0, g1;      // groups of the colour
-            int early_x;     // 1: x is read before the wait on the previous kernel
+            int order;       // among the sweep's launches: 0 the first, 1 the second, 2 a later one
             size_t smem = 0;
         };
         std::vector<Launch> launches;  // in processing order

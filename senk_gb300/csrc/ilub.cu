@@ -252,10 +252,16 @@ __device__ __forceinline__ void sub_slots(T &t, const T (&v)[B][BNW], const T *g
 // that the group's external slots name are gathered into shared memory, warp q
 // subtracts the external slots of step q (their values read straight into
 // registers, a batch of slots ahead), and one warp runs the in-chain part step by
-// step, as k_ilub_sweep does. The staged part (TMA), the first external values
-// and, with early_x, x and the gate are read before the wait on the previous
-// kernel. Same operations in the same order as k_ilub_sweep, which walked a
-// chain's block rows one after another with a dependent gather per four blocks.
+// step, as k_ilub_sweep does. The staged part (TMA) and the first external values
+// are read before the wait on the previous kernel, from the third colour on
+// (order 2; 0 and 1: the first and the second) x and the gate too. The first
+// colour lets the next one start at once, the others after their own wait, so
+// whatever wrote x before the sweep, another plan's sweep included, has completed
+// when the second colour passes its wait. (k_sweep_lv lets every next colour
+// start after its wait and reads x early from the second on; here the colours'
+// CTAs, 2.3 to an SM, then fall up to 5 to an SM instead of 4, 175 us instead of
+// 152.) Same operations in the same order as k_ilub_sweep, which walked a chain's
+// block rows one after another with a dependent gather per four blocks.
 // Block-3x3 system, 48^3 nodes (8 colours), one application: FP64 0.524 ->
 // 0.151 ms, FP32 0.100 ms. It is bound by a colour's dependent steps (a block
 // row's up to 69 FP64 subtractions at 65 cycles, then four in-chain steps) and
@@ -268,8 +274,9 @@ template <typename T> constexpr int bl_min_blocks = sizeof(T) == 8 ? 4 : 0;  // 
 template <typename T, int BNL, int BNW, bool UPPER>
 __global__ void __launch_bounds__(256, bl_min_blocks<T>)
 k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const T *__restrict__ ext,
-              const uint4 *__restrict__ blob, const T *x, T *y, const int *gate, int *status, int early_x)
+              const uint4 *__restrict__ blob, const T *x, T *y, const int *gate, int *status, int order)
 {
+    const bool early_x = order >= 2;
     constexpr int RPW = 32 / BNL, B = bl_batch<T>;
     extern __shared__ __align__(128) unsigned char bls[];
     __shared__ __align__(8) unsigned long long bar;
@@ -290,9 +297,8 @@ k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const 
     if (early_x) {
         for (int i = tid; i < nrows; i += nt) ysh[i] = x[r0 + i];
         skip = gated(gate);
-    } else {
-        pdl_launch_dependents();
     }
+    if (order == 0) pdl_launch_dependents();
     __syncthreads();
     const bool ok = mbar_wait_bounded(&bar, 0, kWaitLimit);
     if (__syncthreads_or(!ok)) {
@@ -324,9 +330,8 @@ k_ilub_slices(const BlGroup *__restrict__ groups, int g0, int per, int n, const 
     int q = w, width = q < per ? wd[q] : 0, k1 = width > 0 ? (width - 1) % B + 1 : 0;
     if (k1 > 0) load(s0, k1);
     pdl_wait();  // the previous colour (or the producer of x) has finished
-    if (early_x) {
-        pdl_launch_dependents();
-    } else {
+    if (order > 0) pdl_launch_dependents();
+    if (!early_x) {
         skip = gated(gate);
         for (int i = tid; i < nrows; i += nt) ysh[i] = x[r0 + i];
     }
@@ -627,7 +632,7 @@ bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, c
     gd.push_back({0, 0, (int)ext, (int)blob});
     for (size_t k = 0; k < F.launches.size(); k++) {
         auto &L = F.launches[k];
-        L.early_x = k > 0;
+        L.order = (int)std::min<size_t>(k, 2);
         for (int g = L.g0; g < L.g1; g++) L.smem = std::max(L.smem, smem[g]);
     }
     F.groups.alloc(gd.size());
@@ -679,7 +684,7 @@ void IlubPlan<T>::sweep(bool upper, const T *x, T *y, cudaStream_t s, const int 
     if (bnl == R && bnw == C)                                                                                  \
         SENK_CUDA(cudaLaunchKernelEx(&cfg, upper ? k_ilub_slices<T, R, C, true> : k_ilub_slices<T, R, C, false>, \
                                      (const BlGroup *)F.groups.p, L.g0, per, n, (const T *)F.ext.p,             \
-                                     (const uint4 *)F.blob.p, x, y, gate, status.p, L.early_x));                \
+                                     (const uint4 *)F.blob.p, x, y, gate, status.p, L.order));                  \
     else
             SENK_ILUB_SHAPES(X)
 #undef X

@@ -1710,13 +1710,12 @@ constexpr int cc_min_blocks(int bs) { return 2048 / (bs * 32) < 32 ? 2048 / (bs 
 //
 // The group's block, its row counts (TMA) and U's inverted diagonal are read
 // before the kernel waits for the previous kernel (programmatic dependent
-// launch). With early_x, x and the gate are read before the wait too and the
-// next kernel may start its prologue only once this one has passed its wait;
-// the host sets it only where the kernels still running cannot be writing
-// these rows (not for the first colour of a sweep; only the sweeps use
-// programmatic launches, so the kernel before a sweep, and every writer of the
-// gate, has completed before its second colour starts). A TMA wait that runs
-// out sets *status = 2.
+// launch). The next kernel may start its prologue once this one has passed its
+// wait, so what runs beside a kernel is its predecessor at most. With early_x,
+// x and the gate are read before the wait too; the host sets it from the second
+// colour of a sweep on: whatever wrote x and the gate, another plan's sweep
+// included, had completed when the first colour passed its wait, and the colour
+// still running writes other rows. A TMA wait that runs out sets *status = 2.
 template <typename VT, typename XT, int BS, bool UPPER>
 __global__ void __launch_bounds__(BS * 32, cc_min_blocks(BS))
 k_sweep_cc(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ chains,
@@ -1764,19 +1763,17 @@ k_sweep_cc(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
         }
         ibase[q] = v - I;
     }
-    // x and the gate: before the wait where early_x allows it (the gate's
-    // writer precedes the sweep), else right after it, so that their loads
-    // overlap the staging wait
+    // x and the gate: before the wait where early_x allows it, else right after
+    // it, so that their loads overlap the staging wait
     XT t = XT(0);
     bool skip = false;
     if (early_x) {
         if (live) t = x[row];
         skip = gated(gate);
     }
-    if (!early_x) pdl_launch_dependents();
     pdl_wait();  // the previous colour (or the producer of x) has finished
-    if (early_x) pdl_launch_dependents();
-    else {
+    pdl_launch_dependents();
+    if (!early_x) {
         skip = gated(gate);
         if (live) t = x[row];
     }
@@ -1861,10 +1858,9 @@ k_sweep_cc2(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__
         }
         skip = gated(gate);
     }
-    if (!early_x) pdl_launch_dependents();
     pdl_wait();  // the previous colour (or the producer of x) has finished
-    if (early_x) pdl_launch_dependents();
-    else {
+    pdl_launch_dependents();
+    if (!early_x) {
         skip = gated(gate);
         if (live) {
             t0 = x[row0];
@@ -1977,15 +1973,12 @@ k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
         for (int r = 0; r < R; r++)
             if (live[r]) t[r] = x[row[r]];
         skip = gated(gate);
-    } else {
-        pdl_launch_dependents();
     }
     pdl_wait();  // the previous colour (or the producer of x) has finished
     // the next colour may start before this one's block has arrived, so that
     // its own is fetched meanwhile
-    if (early_x) {
-        pdl_launch_dependents();
-    } else {
+    pdl_launch_dependents();
+    if (!early_x) {
         skip = gated(gate);
 #pragma unroll
         for (int r = 0; r < R; r++)
@@ -2131,8 +2124,6 @@ k_sweep_lv(const LvGroup *__restrict__ groups, int g0, const uint4 *__restrict__
     if (early_x) {
         for (int i = tid; i < d.nrows; i += nt) ys[i] = x[d.pos0 + i];
         skip = gated(gate);
-    } else {
-        pdl_launch_dependents();
     }
     __syncthreads();
     const bool ok = mbar_wait_bounded(&bar, 0, kWaitLimit);
@@ -2154,9 +2145,8 @@ k_sweep_lv(const LvGroup *__restrict__ groups, int g0, const uint4 *__restrict__
     const uint16_t *place = reinterpret_cast<const uint16_t *>(lvs + P.place);
     const VT *vw = reinterpret_cast<const VT *>(lvs + P.val);
     pdl_wait();  // the previous colour (or the producer of x) has finished
-    if (early_x) {
-        pdl_launch_dependents();
-    } else {
+    pdl_launch_dependents();
+    if (!early_x) {
         skip = gated(gate);
         for (int i = tid; i < d.nrows; i += nt) ys[i] = x[d.pos0 + i];
     }

@@ -305,7 +305,7 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
             typename SweepFactor<VT>::Launch L{};
             L.g0 = lay.colour_groups[c];
             L.g1 = lay.colour_groups[c + 1];
-            L.early_x = c > 0 ? 1 : 0;
+            L.early_x = F.launches.empty() ? 0 : 1;
             L.smem = ((size_t)lay.colour_slots[c] * 32 * (4 + sizeof(VT)) + 32 * (chain_major ? (bs > 16 ? 8 : 4) : 2) * (size_t)bs + 15) / 16 * 16;
             if (L.g1 > L.g0) F.launches.push_back(L);
         }
