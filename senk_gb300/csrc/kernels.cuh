@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "csr_rounds.hpp"
 #include "lv_layout.hpp"
 #include "wf_layout.hpp"
 
@@ -147,24 +148,25 @@ k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const i
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const size_t one = (size_t)(cap + 4) * (sizeof(T) + 4);  // a buffer: values, columns
     unsigned char *buf = csr + 2 * one * wib;
-    const int step = gridDim.x * (blockDim.x >> 5), tiles = (n + 31) >> 5;
+    const int step = gridDim.x * (blockDim.x >> 5), tiles = csr_tiles(n);
     int tile = blockIdx.x * (blockDim.x >> 5) + wib;
     if (tile >= tiles) return;
     const int nnz = __ldg(rptr + n);
     auto bounds = [&](int t, int &a, int &e) {
         const int r = t * 32 + lane;
-        a = t < tiles ? __ldg(rptr + min(r, n)) : 0;
-        e = t < tiles ? __ldg(rptr + min(r + 1, n)) : 0;
+        a = t < tiles ? __ldg(rptr + csr_begin_at(r, n)) : 0;
+        e = t < tiles ? __ldg(rptr + csr_end_at(r, n)) : 0;
     };
     // entries [c0, c0 + cap) of the tile that ends at s1 into buffer k; c0 is
     // rounded down to a multiple of 4
     auto fetch = [&](int k, int c0, int s1) {
         T *sv = reinterpret_cast<T *>(buf + k * one);
         int *sc = reinterpret_cast<int *>(sv + cap + 4);
-        const int cnt = min(cap, s1 - c0);
+        const int cnt = csr_round(c0, cap, s1);
         for (int i = lane * EV; i < cnt; i += 32 * EV)
-            cp_async16(sv + i, val + c0 + i, min(16, (nnz - c0 - i) * (int)sizeof(T)));
-        for (int i = lane * 4; i < cnt; i += 128) cp_async16(sc + i, cind + c0 + i, min(16, (nnz - c0 - i) * 4));
+            cp_async16(sv + i, val + c0 + i, csr_piece_bytes(c0 + i, nnz, (int)sizeof(T)));
+        for (int i = lane * 4; i < cnt; i += 128)
+            cp_async16(sc + i, cind + c0 + i, csr_piece_bytes(c0 + i, nnz, 4));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     int a, e, a1, e1, k = 0;
@@ -175,11 +177,11 @@ k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const i
     T sum[S] = {};
     for (;;) {
         // the next round: the rest of this tile, or the next tile
-        const bool more = c0 + cap < s1;
-        int d0 = c0 + cap, t1 = s1;
-        if (!more) {
-            d0 = __shfl_sync(0xffffffffu, a1, 0) & ~3;
-            t1 = __shfl_sync(0xffffffffu, e1, 31);
+        const bool more = csr_more(c0, cap, s1);
+        int d0 = __shfl_sync(0xffffffffu, a1, 0) & ~3, t1 = __shfl_sync(0xffffffffu, e1, 31);
+        if (more) {
+            d0 = c0 + cap;
+            t1 = s1;
         }
         const bool any = more || tile + step < tiles;
         if (any) fetch(k ^ 1, d0, t1);

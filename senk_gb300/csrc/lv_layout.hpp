@@ -84,10 +84,12 @@ static_assert(sizeof(LvRecord) == 8, "LvRecord is one 8-byte load");
 struct LvParts {
     unsigned first, rows, rec, cols, dinv, place, val, end;
 };
+#ifndef SENK_HD
 #ifdef __CUDACC__
 #define SENK_HD __host__ __device__
 #else
 #define SENK_HD
+#endif
 #endif
 SENK_HD constexpr unsigned lv_round(unsigned b) { return (b + 15u) / 16u * 16u; }
 SENK_HD constexpr LvParts lv_parts(const LvHeader &h, unsigned dinv_bytes, unsigned vb)
