@@ -69,7 +69,8 @@ size_t wf_bytes_for(int slots, int bs, bool upper)
 // What a lane of k_sweep_rl needs of its row: the external entries of the
 // chain's rows solved before it (eo) and its own (ne), the same of in-chain
 // entries (io, left), and the levels of its chain. Chains of up to 16 rows take
-// one word (io <= 120 and left, depth <= 15 there), longer ones two.
+// one word (with distinct columns io <= 120 and left, depth <= 15 there; the
+// builder checks them, as columns may be repeated), longer ones two.
 struct RowWord {
     int eo, ne, io, left, depth;
 };
@@ -265,7 +266,7 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
                     const unsigned ne = cnt[l], left = cnt[bs + l];
                     unsigned *w = &out.rows[(((size_t)g * 32 + q) * bs + l) * rw];
                     if (rw == 1) {
-                        packs = packs && eo < 1024 && ne < 128;
+                        packs = packs && eo < 1024 && ne < 128 && io < 128 && left < 16;
                         *w = eo | ne << 10 | io << 17 | left << 24 | depth << 28;
                     } else {
                         w[0] = eo | ne << 16 | depth << 24;
