@@ -242,19 +242,21 @@ __device__ __forceinline__ void cta_sum_columns(const double *part, int P, int n
 // Every CTA writes its partials, fences, and bumps a ticket; the CTA that draws
 // the last ticket sees all partials and finalizes (then resets the ticket so the
 // same counter serves the next launch, including inside a replayed CUDA graph).
-__device__ __forceinline__ bool last_cta_arrives(unsigned int *ticket, unsigned int total)
+// RESET = false: the counter runs on; this launch's tickets start at `first`.
+template <bool RESET = true>
+__device__ __forceinline__ bool last_cta_arrives(unsigned int *ticket, unsigned int total, unsigned int first = 0)
 {
     __shared__ bool is_last;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned int t = atomicAdd(ticket, 1u);
-        is_last = (t == total - 1);
+        is_last = (t - first == total - 1);
     }
     __syncthreads();
     if (is_last) {
         __threadfence();
-        if (threadIdx.x == 0) *ticket = 0;
+        if (RESET && threadIdx.x == 0) *ticket = 0;
     }
     return is_last;
 }

@@ -458,10 +458,17 @@ __device__ __forceinline__ void dot_columns(const XT *__restrict__ V, long long 
 // addition in use (65 instructions for 8 columns; warp reductions took 360),
 // and the launcher keeps the CTAs to one wave over all chunks.
 // 30 columns of 2.1M rows: 178 -> 132 us; 1 column 17 -> 14 us.
-template <typename XT, bool ACCUM>
+//
+// HOST: coef is host memory that the host polls. As soon as it sees the result it
+// may launch the next reduction, on another stream too, and nothing orders a
+// store of this kernel before that. So the ticket is not reset but counts on from
+// `first`, which the host keeps: the last CTA's ticket shows that all additions to
+// it have been made, and the partials have been read when their sum is stored. (A
+// reset with a system-wide fence before the result costs 0.3 us of a 10 us dot.)
+template <typename XT, bool ACCUM, bool HOST = false>
 __global__ void __launch_bounds__(kThreads)
 k_multidot(const XT *__restrict__ V, long long ldv, int nv, const XT *__restrict__ w, long long n,
-           double *part, unsigned *ticket, double *coef, double *hcol, const int *gate)
+           double *part, unsigned *ticket, double *coef, double *hcol, const int *gate, unsigned first = 0)
 {
     if (gated(gate)) return;
     constexpr int CH = 8;
@@ -509,7 +516,7 @@ k_multidot(const XT *__restrict__ V, long long ldv, int nv, const XT *__restrict
         if ((int)threadIdx.x < nc) part[(long long)(c0 + threadIdx.x) * gridDim.x + blockIdx.x] = sh[threadIdx.x][0];
     }
     const unsigned total = gridDim.x * gridDim.y;
-    if (last_cta_arrives(ticket, total)) {
+    if (last_cta_arrives<!HOST>(ticket, total, first)) {
         __shared__ double shp[32];
         cta_sum_columns(part, gridDim.x, nv, shp, [&](int k, double s) {
             coef[k] = s;

@@ -300,9 +300,10 @@ std::mutex g_red_mu;
 ReduceScratch g_red[64];
 
 // The result's place in pinned host memory that the kernel writes itself, per
-// device (kept for the life of the process).
+// device (kept for the life of the process), and the tickets drawn so far.
 double *g_red_host[64];
 double *g_red_host_dev[64];
+unsigned g_red_drawn[64];
 
 // A signalling NaN that no reduction returns: the place holds it until the
 // kernel has written.
@@ -311,15 +312,21 @@ constexpr unsigned long long kNoResult = 0x7ff4a5a5c3c35a5aull;
 // Waits for the result of the reduction launched on s: a few hundred
 // microseconds of reading its place (a dot product of a small system takes
 // less than a copy and a synchronisation, 10 us), then the stream, whose
-// errors are reported.
-double wait_result(const double *place, cudaStream_t s)
+// errors are reported. A kernel that ended without a result found another
+// number of tickets drawn than `drawn`, after a call that failed: the count
+// starts anew.
+double wait_result(const double *place, ReduceScratch &red, unsigned &drawn, cudaStream_t s)
 {
     const volatile unsigned long long *bits = reinterpret_cast<const volatile unsigned long long *>(place);
     const auto give_up = std::chrono::steady_clock::now() + std::chrono::microseconds(300);
     while (*bits == kNoResult)
         if (std::chrono::steady_clock::now() > give_up) {
             SENK_CUDA(cudaStreamSynchronize(s));
-            break;
+            if (*bits != kNoResult) break;
+            SENK_CUDA(cudaMemsetAsync(red.ticket.p, 0, sizeof(unsigned), s));
+            SENK_CUDA(cudaStreamSynchronize(s));
+            drawn = 0;
+            throw CudaError{cudaErrorUnknown, "reduction without a result", __FILE__, __LINE__};
         }
     std::atomic_thread_fence(std::memory_order_acquire);
     return *const_cast<const volatile double *>(place);
@@ -420,11 +427,12 @@ static int dev_reduce(const char *fn, const double *x, const double *y, int N, d
         }
         *reinterpret_cast<volatile unsigned long long *>(g_red_host[dev]) = kNoResult;
         const int grid = stream_grid(N, kThreads, 2);
-        k_multidot<double, false><<<dim3(grid, 1), kThreads, 0, s>>>(x, 0, 1, y, N, g_red[dev].part.p,
-                                                                     g_red[dev].ticket.p, g_red_host_dev[dev], nullptr,
-                                                                     nullptr);
+        k_multidot<double, false, true><<<dim3(grid, 1), kThreads, 0, s>>>(x, 0, 1, y, N, g_red[dev].part.p,
+                                                                           g_red[dev].ticket.p, g_red_host_dev[dev],
+                                                                           nullptr, nullptr, g_red_drawn[dev]);
         SENK_LAUNCH_CHECK();
-        const double h = wait_result(g_red_host[dev], s);
+        const double h = wait_result(g_red_host[dev], g_red[dev], g_red_drawn[dev], s);
+        g_red_drawn[dev] += (unsigned)grid;
         *result = norm ? sqrt(h) : h;
         return (int)kOk;
     });
