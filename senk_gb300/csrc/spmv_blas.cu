@@ -24,6 +24,10 @@ namespace {
 // against 101, FP32 51 against 33 (few warps' buffers fit an SM then).
 constexpr int kRowsMean = 40;
 
+// Shared memory that an SM's warps of k_spmv_csr_rows may take; a CTA takes a
+// quarter of it at most (one warp, of at most 36 KB, where fewer than 8 fit).
+constexpr size_t kRowsSmem = 220 * 1024;
+
 template <typename T, int MODE>
 void spmv_csr_rows(const T *v, const int *c, const int *r, const T *x, const T *b, T *y, int n, long long nnz,
                    cudaStream_t s, const int *gate)
@@ -32,13 +36,16 @@ void spmv_csr_rows(const T *v, const int *c, const int *r, const T *x, const T *
     const int mean = (int)((nnz + n - 1) / n);
     const int cap = std::max(256, (mean * 36 + 63) / 64 * 64);
     const size_t per_warp = 2 * (size_t)(cap + 4) * (sizeof(T) + 4);
-    const int resident = (int)std::min<size_t>(32, (size_t)220 * 1024 / per_warp);  // warps per SM
+    const int resident = (int)std::min<size_t>(32, kRowsSmem / per_warp);  // warps per SM
     const int warps = resident >= 16 ? 4 : resident >= 8 ? 2 : 1;
     const int tiles = ceil_div(n, 32);
     const int grid = std::min(ceil_div(tiles, warps), resident / warps * sm_count());
     const size_t smem = per_warp * warps;
+    // the same limit for every matrix: it belongs to the function, and another
+    // thread's call may come between it and the launch
     if (smem > 48 * 1024)
-        SENK_CUDA(cudaFuncSetAttribute(k_spmv_csr_rows<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SENK_CUDA(cudaFuncSetAttribute(k_spmv_csr_rows<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kRowsSmem / 4));
     k_spmv_csr_rows<T, MODE><<<grid, warps * 32, smem, s>>>(v, c, r, x, b, y, n, cap, gate);
 }
 
