@@ -86,27 +86,126 @@ k_spmv_csr(const MT *__restrict__ val, const int *__restrict__ cind, const int *
     }
 }
 
-// sum += v[u] * xv[u] for the last n of 8 slots (n the same in the whole warp).
-// FP64 enters the chain by a jump, in order (a predicated FP64 instruction
-// costs as much as one that runs, see sub_last); FP32 adds into four sums.
-template <typename T, int S>
-__device__ __forceinline__ void add_last8(T (&sum)[S], const T (&v)[8], const T (&xv)[8], int n)
+// Row sums of k_spmv_csr_rows. Their rounding may not exceed that of k_spmv_csr,
+// which takes 2 to 32 lanes a row and a tree over them. Root mean square of the
+// error over that kernel's, on random rows and on rows with a dominant middle:
+//     entries                     5      7      8      27     40     48     64
+//     one running sum         0.89   0.95   1.00   1.46   1.71   1.84   2.12
+//                             0.94   1.09   0.98   1.67   1.80
+//     four sums               0.97   0.93   0.93   0.98   1.06   1.11   1.24
+//                             0.99   0.98   0.88   1.08   1.09
+//     eight sums, as a tree   1.00   1.00   1.00   0.94   0.96   0.99   1.05
+//                             1.00   1.00   1.00   1.00   1.00
+//     two sums in tree order  0.88   0.90   0.90
+//                             0.83   0.82   0.98
+// (the 7-point convection-diffusion rows: one sum 1.14, four 1.00, two in tree order
+// 0.85; 5-point rows: 1.23, 1.00, 1.00). In FP64 an addition more is 14 % of a
+// 7-entry row, so rows of up to 8 entries take the two sums and longer ones eight.
+constexpr int kRowTwo = 8;
+
+// The products of slots [0, M) in the order of a tree over eight lanes: slots 0, 4,
+// 2, 6 in one sum, 1, 5, 3, 7 in the other.
+template <int M, typename T>
+__device__ __forceinline__ void add_two(T &even, T &odd, const T (&v)[8], const T (&xv)[8])
 {
-    if constexpr (S == 1) {
-        switch (n) {
-        case 8: sum[0] += v[0] * xv[0];
-        case 7: sum[0] += v[1] * xv[1];
-        case 6: sum[0] += v[2] * xv[2];
-        case 5: sum[0] += v[3] * xv[3];
-        case 4: sum[0] += v[4] * xv[4];
-        case 3: sum[0] += v[5] * xv[5];
-        case 2: sum[0] += v[6] * xv[6];
-        case 1: sum[0] += v[7] * xv[7];
+    even += v[0] * xv[0];
+    if constexpr (M > 4) even += v[4] * xv[4];
+    if constexpr (M > 2) even += v[2] * xv[2];
+    if constexpr (M > 6) even += v[6] * xv[6];
+    if constexpr (M > 1) odd += v[1] * xv[1];
+    if constexpr (M > 5) odd += v[5] * xv[5];
+    if constexpr (M > 3) odd += v[3] * xv[3];
+    if constexpr (M > 7) odd += v[7] * xv[7];
+}
+
+// The first m of 8 slots (m the same in the whole warp). FP64 jumps to the code for
+// m slots (a predicated FP64 instruction costs as much as one that runs, see
+// sub_last); in FP32 the other slots add zero.
+template <typename T>
+__device__ __forceinline__ void add_two(T &even, T &odd, const T (&v)[8], const T (&xv)[8], int m)
+{
+    if constexpr (sizeof(T) == 8) {
+        switch (m) {
+        case 8: add_two<8>(even, odd, v, xv); break;
+        case 7: add_two<7>(even, odd, v, xv); break;
+        case 6: add_two<6>(even, odd, v, xv); break;
+        case 5: add_two<5>(even, odd, v, xv); break;
+        case 4: add_two<4>(even, odd, v, xv); break;
+        case 3: add_two<3>(even, odd, v, xv); break;
+        case 2: add_two<2>(even, odd, v, xv); break;
+        case 1: add_two<1>(even, odd, v, xv); break;
+        default: break;
+        }
+    } else {
+        add_two<8>(even, odd, v, xv);
+    }
+}
+
+// sum[u] += v[u] * xv[u] for the first m of 8 slots, as above.
+template <typename T>
+__device__ __forceinline__ void add_eight(T (&sum)[8], const T (&v)[8], const T (&xv)[8], int m)
+{
+    if constexpr (sizeof(T) == 8) {
+        switch (m) {
+        case 8: sum[7] += v[7] * xv[7];
+        case 7: sum[6] += v[6] * xv[6];
+        case 6: sum[5] += v[5] * xv[5];
+        case 5: sum[4] += v[4] * xv[4];
+        case 4: sum[3] += v[3] * xv[3];
+        case 3: sum[2] += v[2] * xv[2];
+        case 2: sum[1] += v[1] * xv[1];
+        case 1: sum[0] += v[0] * xv[0];
         default: break;
         }
     } else {
 #pragma unroll
-        for (int u = 0; u < 8; u++) sum[u % S] += v[u] * xv[u];
+        for (int u = 0; u < 8; u++) sum[u] += v[u] * xv[u];
+    }
+}
+
+// A lane's sums of its row of a tile with rows of more than kRowTwo entries.
+template <typename T>
+struct CsrSums {
+    T sum[8];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int u = 0; u < 8; u++) sum[u] = T(0);
+    }
+    __device__ __forceinline__ T tree() const
+    {
+        return ((sum[0] + sum[4]) + (sum[2] + sum[6])) + ((sum[1] + sum[5]) + (sum[3] + sum[7]));
+    }
+};
+
+// Slots [0, 8) of a lane's len staged entries (columns sc, values sv) from k0 on;
+// those past len are zero. All gathers of x are issued before the first is used.
+template <typename T>
+__device__ __forceinline__ void csr_slots(const T *sv, const int *sc, const T *__restrict__ x, int k0, int len,
+                                          T (&v)[8], T (&xv)[8])
+{
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        v[u] = T(0);
+        xv[u] = T(0);
+        if (k0 + u < len) {
+            xv[u] = __ldg(x + sc[k0 + u]);
+            v[u] = sv[k0 + u];
+        }
+    }
+}
+
+// One round (cap entries from c0 on) of such a tile, this lane's row being [a, e).
+template <typename T>
+__device__ __forceinline__ void csr_add_round(CsrSums<T> &st, const T *sv, const int *sc, const T *__restrict__ x, int a,
+                                              int e, int c0, int cap)
+{
+    const int lo = max(a - c0, 0), len = min(e - c0, cap) - lo;
+    const int longest = __reduce_max_sync(0xffffffffu, len);
+    for (int k0 = 0; k0 < longest; k0 += 8) {
+        T v[8], xv[8];
+        csr_slots(sv + lo, sc + lo, x, k0, len, v, xv);
+        add_eight(st.sum, v, xv, min(8, longest - k0));
     }
 }
 
@@ -117,32 +216,17 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, int valid
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid) : "memory");
 }
 
-// CSR SpMV of short rows: one warp takes 32 consecutive rows at a time, whose
-// entries are consecutive, copies them to shared memory (cp.async, 16 bytes a
-// lane, the next 32 rows' while these are added), and every lane adds one row
-// with its x gathers issued eight at a time. Neighbouring rows have
-// neighbouring columns, so a gather of 32 rows falls in few sectors.
-//
-// FP64 is why: the unit takes one warp instruction in 19 cycles per SM, and
-// G lanes per row (k_spmv_csr) spend log2(G) additions for 32 / G rows besides
-// the products; here a warp's FP64 instructions are its 32 rows' longest row.
-// Rows are added in column order in FP64 and into four sums in FP32 (one
-// running sum would round more than the lanes did).
-//
-// 7-point rows: FP64 128^3 158 -> 41 us (5.3 TB/s), FP32 128^3 59 -> 30 us
-// (4.8 TB/s); 27-point rows on 96^3 FP64 345 -> 89 us, FP32 95 -> 49 us (before:
-// k_spmv_csr). Its copies and sums share the SM with 32 warps, so what is left
-// is FP64's 28 us and the bytes' 32 us at 128^3 not overlapping entirely.
-//
-// val and cind 16-byte aligned. cap: entries a buffer holds (a multiple of 4);
-// 32 rows with more take several rounds. MODE 0: y = A x; MODE 1: y = b - A x.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(128, 8)
-k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const int *__restrict__ rptr,
-                const T *__restrict__ x, const T *__restrict__ b, T *__restrict__ y, int n, int cap, const int *gate)
+// The tiles of k_spmv_csr_rows that a pass adds: all of them, those whose rows are
+// all short (kRowTwo), or the others.
+constexpr int kCsrAll = 0, kCsrShort = 1, kCsrOthers = 2;
+
+// One pass over the warp's tiles; returns whether it left some out. A tile that is
+// left out counts as empty and is not copied.
+template <typename T, int MODE, int TILES>
+__device__ __forceinline__ bool csr_rows_pass(const T *__restrict__ val, const int *__restrict__ cind,
+                                              const int *__restrict__ rptr, const T *__restrict__ x,
+                                              const T *__restrict__ b, T *__restrict__ y, int n, int cap)
 {
-    if (gated(gate)) return;
-    constexpr int S = sizeof(T) == 4 ? 4 : 1;
     constexpr int EV = 16 / (int)sizeof(T);  // entries of a 16-byte piece of val
     extern __shared__ __align__(16) unsigned char csr[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -150,12 +234,17 @@ k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const i
     unsigned char *buf = csr + 2 * one * wib;
     const int step = gridDim.x * (blockDim.x >> 5), tiles = csr_tiles(n);
     int tile = blockIdx.x * (blockDim.x >> 5) + wib;
-    if (tile >= tiles) return;
+    if (tile >= tiles) return false;
     const int nnz = __ldg(rptr + n);
     auto bounds = [&](int t, int &a, int &e) {
         const int r = t * 32 + lane;
         a = t < tiles ? __ldg(rptr + csr_begin_at(r, n)) : 0;
         e = t < tiles ? __ldg(rptr + csr_end_at(r, n)) : 0;
+    };
+    // whether the pass adds the tile whose rows are [a, e)
+    auto taken = [&](int a, int e) {
+        if constexpr (TILES == kCsrAll) return true;
+        else return __all_sync(0xffffffffu, e - a <= kRowTwo) == (TILES == kCsrShort);
     };
     // entries [c0, c0 + cap) of the tile that ends at s1 into buffer k; c0 is
     // rounded down to a multiple of 4
@@ -169,16 +258,28 @@ k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const i
             cp_async16(sc + i, cind + c0 + i, csr_piece_bytes(c0 + i, nnz, 4));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int a, e, a1, e1, k = 0;
+    // the first entry copied and the last one of the tile with rows [a, e)
+    auto range = [&](int a, int e, bool take, int &c0, int &s1) {
+        c0 = __shfl_sync(0xffffffffu, a, 0) & ~3;
+        s1 = __shfl_sync(0xffffffffu, e, 31);
+        if (!take) s1 = c0;
+    };
+    bool left_out = false;
+    int a, e, a1, e1, c0, s1, k = 0;
     bounds(tile, a, e);
     bounds(tile + step, a1, e1);
-    int c0 = __shfl_sync(0xffffffffu, a, 0) & ~3, s1 = __shfl_sync(0xffffffffu, e, 31);
+    bool take = taken(a, e);
+    range(a, e, take, c0, s1);
     fetch(0, c0, s1);
-    T sum[S] = {};
+    T even = T(0), odd = T(0);
+    CsrSums<T> st;
+    if constexpr (TILES != kCsrShort) st.clear();
     for (;;) {
         // the next round: the rest of this tile, or the next tile
         const bool more = csr_more(c0, cap, s1);
-        int d0 = __shfl_sync(0xffffffffu, a1, 0) & ~3, t1 = __shfl_sync(0xffffffffu, e1, 31);
+        const bool take1 = taken(a1, e1);
+        int d0, t1;
+        range(a1, e1, take1, d0, t1);
         if (more) {
             d0 = c0 + cap;
             t1 = s1;
@@ -190,39 +291,85 @@ k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const i
         __syncwarp();
         const T *sv = reinterpret_cast<const T *>(buf + k * one);
         const int *sc = reinterpret_cast<const int *>(sv + cap + 4);
-        const int lo = max(a - c0, 0), len = min(e - c0, cap) - lo;
-        const int longest = __reduce_max_sync(0xffffffffu, len);
-        for (int k0 = 0; k0 < longest; k0 += 8) {
-            const int m = min(8, longest - k0), f = k0 - (8 - m);
-            T v[8], xv[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                v[u] = T(0);
-                xv[u] = T(0);
-                if (f + u >= k0 && f + u < len) {
-                    xv[u] = __ldg(x + sc[lo + f + u]);
-                    v[u] = sv[lo + f + u];
-                }
+        if (take) {
+            if constexpr (TILES == kCsrShort) {
+                const int lo = max(a - c0, 0), len = min(e - c0, cap) - lo;
+                T v[8], xv[8];
+                csr_slots(sv + lo, sc + lo, x, 0, len, v, xv);
+                add_two(even, odd, v, xv, __reduce_max_sync(0xffffffffu, len));
+            } else {
+                csr_add_round(st, sv, sc, x, a, e, c0, cap);
             }
-            add_last8<T, S>(sum, v, xv, m);
         }
         __syncwarp();  // buffer k may be filled again
         if (!more) {
             const int row = tile * 32 + lane;
-            if constexpr (S == 4) sum[0] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            if (row < n) y[row] = MODE == 1 ? b[row] - sum[0] : sum[0];
-#pragma unroll
-            for (int u = 0; u < S; u++) sum[u] = T(0);
+            if (take) {
+                const T t = TILES == kCsrShort ? even + odd : st.tree();
+                if (row < n) y[row] = MODE == 1 ? b[row] - t : t;
+                even = odd = T(0);
+                if constexpr (TILES != kCsrShort) st.clear();
+            }
+            left_out |= !take;
             tile += step;
-            if (tile >= tiles) return;
+            if (tile >= tiles) return left_out;
             a = a1;
             e = e1;
+            take = take1;
             bounds(tile + step, a1, e1);
         }
         c0 = d0;
         s1 = t1;
         k ^= 1;
     }
+}
+
+// The pass over the tiles with longer rows, called once at the end: inlined, it
+// takes registers from the loop over the short ones (45 us for 43).
+template <typename T, int MODE>
+__device__ __noinline__ void csr_rows_others(const T *__restrict__ val, const int *__restrict__ cind,
+                                             const int *__restrict__ rptr, const T *__restrict__ x,
+                                             const T *__restrict__ b, T *__restrict__ y, int n, int cap)
+{
+    csr_rows_pass<T, MODE, kCsrOthers>(val, cind, rptr, x, b, y, n, cap);
+}
+
+// Warps per SM that k_spmv_csr_rows is compiled for: 64 registers a thread, 85 in
+// FP64 with LONG, whose buffers let 24 warps in. (28 warps in FP64 without LONG: rows
+// of 0 to 14 entries, added in the second pass, 114 instead of 146 us, but 7-entry
+// rows 44 instead of 43.)
+template <typename T, bool LONG>
+constexpr int csr_rows_warps = LONG && sizeof(T) == 8 ? 24 : 32;
+
+// CSR SpMV of short rows: one warp takes 32 consecutive rows at a time, whose
+// entries are consecutive, copies them to shared memory (cp.async, 16 bytes a
+// lane, the next 32 rows' while these are added), and every lane adds one row
+// with its x gathers issued eight at a time. Neighbouring rows have
+// neighbouring columns, so a gather of 32 rows falls in few sectors.
+//
+// FP64 is why: the unit takes one warp instruction in 19 cycles per SM, and
+// G lanes per row (k_spmv_csr) spend log2(G) additions for 32 / G rows besides
+// the products; here a warp's FP64 instructions are its 32 rows' longest row.
+// A tile of short rows (kRowTwo) adds them at once, another by csr_add_round: in
+// a second pass where short rows are the rule, so that its registers are not
+// theirs (both in one loop: 48 us for 43), or all tiles so (LONG).
+//
+// 7-point rows: FP64 128^3 158 -> 43 us (5.1 TB/s), FP32 128^3 59 -> 30 us
+// (4.8 TB/s); 27-point rows on 96^3 FP64 345 -> 89 us, FP32 95 -> 49 us (before:
+// k_spmv_csr). Its copies and sums share the SM with 32 warps, so what is left
+// is FP64's 32 us and the bytes' 32 us at 128^3 not overlapping entirely.
+//
+// val and cind 16-byte aligned. cap: entries a buffer holds (a multiple of 4);
+// 32 rows with more take several rounds. MODE 0: y = A x; MODE 1: y = b - A x.
+template <typename T, int MODE, bool LONG>
+__global__ void __launch_bounds__(128, csr_rows_warps<T, LONG> / 4)
+k_spmv_csr_rows(const T *__restrict__ val, const int *__restrict__ cind, const int *__restrict__ rptr,
+                const T *__restrict__ x, const T *__restrict__ b, T *__restrict__ y, int n, int cap, const int *gate)
+{
+    if (gated(gate)) return;
+    if constexpr (LONG) csr_rows_pass<T, MODE, kCsrAll>(val, cind, rptr, x, b, y, n, cap);
+    else if (csr_rows_pass<T, MODE, kCsrShort>(val, cind, rptr, x, b, y, n, cap))
+        csr_rows_others<T, MODE>(val, cind, rptr, x, b, y, n, cap);
 }
 
 // Row sum of one SELL-32 row (lane r of the slice at element offset o, w

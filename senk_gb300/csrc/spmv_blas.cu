@@ -28,15 +28,15 @@ constexpr int kRowsMean = 40;
 // quarter of it at most (one warp, of at most 36 KB, where fewer than 8 fit).
 constexpr size_t kRowsSmem = 220 * 1024;
 
-template <typename T, int MODE>
-void spmv_csr_rows(const T *v, const int *c, const int *r, const T *x, const T *b, T *y, int n, long long nnz,
-                   cudaStream_t s, const int *gate)
+template <typename T, int MODE, bool LONG>
+void spmv_csr_rows_as(const T *v, const int *c, const int *r, const T *x, const T *b, T *y, int n, long long nnz,
+                      cudaStream_t s, const int *gate)
 {
     // a buffer holds 32 rows an eighth longer than the mean
     const int mean = (int)((nnz + n - 1) / n);
     const int cap = std::max(256, (mean * 36 + 63) / 64 * 64);
     const size_t per_warp = 2 * (size_t)(cap + 4) * (sizeof(T) + 4);
-    const int resident = (int)std::min<size_t>(32, kRowsSmem / per_warp);  // warps per SM
+    const int resident = (int)std::min<size_t>(csr_rows_warps<T, LONG>, kRowsSmem / per_warp);  // warps per SM
     const int warps = resident >= 16 ? 4 : resident >= 8 ? 2 : 1;
     const int tiles = ceil_div(n, 32);
     const int grid = std::min(ceil_div(tiles, warps), resident / warps * sm_count());
@@ -44,9 +44,19 @@ void spmv_csr_rows(const T *v, const int *c, const int *r, const T *x, const T *
     // the same limit for every matrix: it belongs to the function, and another
     // thread's call may come between it and the launch
     if (smem > 48 * 1024)
-        SENK_CUDA(cudaFuncSetAttribute(k_spmv_csr_rows<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        SENK_CUDA(cudaFuncSetAttribute(k_spmv_csr_rows<T, MODE, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kRowsSmem / 4));
-    k_spmv_csr_rows<T, MODE><<<grid, warps * 32, smem, s>>>(v, c, r, x, b, y, n, cap, gate);
+    k_spmv_csr_rows<T, MODE, LONG><<<grid, warps * 32, smem, s>>>(v, c, r, x, b, y, n, cap, gate);
+}
+
+// The line between the two forms: FP64 rows of 8 entries 62 us in two sums, 70 all
+// tiles by csr_add_round; of 9, 70 in two passes, 40 in one (FP32 46, 46; 27, 25).
+template <typename T, int MODE>
+void spmv_csr_rows(const T *v, const int *c, const int *r, const T *x, const T *b, T *y, int n, long long nnz,
+                   cudaStream_t s, const int *gate)
+{
+    if (nnz <= (long long)kRowTwo * n) spmv_csr_rows_as<T, MODE, false>(v, c, r, x, b, y, n, nnz, s, gate);
+    else spmv_csr_rows_as<T, MODE, true>(v, c, r, x, b, y, n, nnz, s, gate);
 }
 
 template <typename MT, typename XT, int MODE>
