@@ -101,7 +101,10 @@ k_spmv_csr(const MT *__restrict__ val, const int *__restrict__ cind, const int *
 // (the 7-point convection-diffusion rows: one sum 1.14, four 1.00, two in tree order
 // 0.85; 5-point rows: 1.23, 1.00, 1.00). In FP64 an addition more is 14 % of a
 // 7-entry row, so rows of up to 8 entries take the two sums and longer ones eight.
-constexpr int kRowTwo = 8;
+// Rows of more than 48 entries take 32 sums, over several lanes (one lane took 6.1
+// ms for a row of 100,000 FP64 entries among 7-entry rows, now the call takes 1.3;
+// k_spmv_csr 4.6).
+constexpr int kRowTwo = 8, kRowMost = 48;
 
 // The products of slots [0, M) in the order of a tree over eight lanes: slots 0, 4,
 // 2, 6 in one sum, 1, 5, 3, 7 in the other.
@@ -167,15 +170,19 @@ __device__ __forceinline__ void add_eight(T (&sum)[8], const T (&v)[8], const T 
 template <typename T>
 struct CsrSums {
     T sum[8];
+    T total;  // of a long row
+    T part;   // this lane's part of a long row that goes on in the next round
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
         for (int u = 0; u < 8; u++) sum[u] = T(0);
+        total = part = T(0);
     }
     __device__ __forceinline__ T tree() const
     {
         return ((sum[0] + sum[4]) + (sum[2] + sum[6])) + ((sum[1] + sum[5]) + (sum[3] + sum[7]));
     }
+    __device__ __forceinline__ T row(int entries) const { return entries > kRowMost ? total : tree(); }
 };
 
 // Slots [0, 8) of a lane's len staged entries (columns sc, values sv) from k0 on;
@@ -200,12 +207,65 @@ template <typename T>
 __device__ __forceinline__ void csr_add_round(CsrSums<T> &st, const T *sv, const int *sc, const T *__restrict__ x, int a,
                                               int e, int c0, int cap)
 {
-    const int lo = max(a - c0, 0), len = min(e - c0, cap) - lo;
+    const int lane = threadIdx.x & 31;
+    const bool big = e - a > kRowMost;
+    const int lo = max(a - c0, 0), len = big ? 0 : min(e - c0, cap) - lo;
     const int longest = __reduce_max_sync(0xffffffffu, len);
     for (int k0 = 0; k0 < longest; k0 += 8) {
         T v[8], xv[8];
         csr_slots(sv + lo, sc + lo, x, k0, len, v, xv);
         add_eight(st.sum, v, xv, min(8, longest - k0));
+    }
+    // long rows, 32 sums and a tree each. Those that lie in this round: four at a
+    // time, eight lanes a row with four sums
+    const bool within = big && a >= c0 && e - c0 <= cap;
+    const unsigned rows = __ballot_sync(0xffffffffu, within);
+    const int rank = __popc(rows & ((1u << lane) - 1u));
+    unsigned m = rows;
+    for (int four = 0; m; four++) {
+        int q = -1;  // the row of this lane's eight lanes; -1: none left
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (lane >> 3 == u) q = __ffs(m) - 1;
+            m &= m - 1;
+        }
+        const int qa = __shfl_sync(0xffffffffu, a, q & 31), qe = __shfl_sync(0xffffffffu, e, q & 31);
+        const int first = qa - c0, qn = q >= 0 ? qe - qa : 0, most = __reduce_max_sync(0xffffffffu, qn);
+        T p[4] = {};
+        for (int k0 = lane & 7; k0 < most; k0 += 32) {
+            T v[4], xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                v[u] = T(0);
+                xv[u] = T(0);
+                if (k0 + 8 * u < qn) {
+                    xv[u] = __ldg(x + sc[first + k0 + 8 * u]);
+                    v[u] = sv[first + k0 + 8 * u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) p[u] += v[u] * xv[u];
+        }
+        __syncwarp();
+        T t = (p[0] + p[2]) + (p[1] + p[3]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        t = __shfl_sync(0xffffffffu, t, 8 * (rank & 3));
+        if (within && rank >> 2 == four) st.total = t;
+    }
+    // those that reach past this round, by the whole warp: the entries of all rows
+    // are in order, so at most one comes from the round before and one goes on
+    for (unsigned m = __ballot_sync(0xffffffffu, big && !within && e > c0 && a - c0 < cap); m; m &= m - 1) {
+        const int q = __ffs(m) - 1, qe = __shfl_sync(0xffffffffu, e, q);
+        const int first = max(__shfl_sync(0xffffffffu, a, q) - c0, 0), end = min(qe - c0, cap);
+#pragma unroll 4
+        for (int i = first + lane; i < end; i += 32) st.part += sv[i] * __ldg(x + sc[i]);
+        __syncwarp();
+        if (qe - c0 <= cap) {
+            const T t = warp_sum(st.part);
+            if (lane == q) st.total = t;
+            st.part = T(0);
+        }
     }
 }
 
@@ -305,7 +365,7 @@ __device__ __forceinline__ bool csr_rows_pass(const T *__restrict__ val, const i
         if (!more) {
             const int row = tile * 32 + lane;
             if (take) {
-                const T t = TILES == kCsrShort ? even + odd : st.tree();
+                const T t = TILES == kCsrShort ? even + odd : st.row(e - a);
                 if (row < n) y[row] = MODE == 1 ? b[row] - t : t;
                 even = odd = T(0);
                 if constexpr (TILES != kCsrShort) st.clear();

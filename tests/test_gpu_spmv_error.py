@@ -40,3 +40,23 @@ def _errors(lens, dtype, seed):
 def test_rows_of_one_length(per, dtype):
     rows, general = _errors(np.full(100_000, per), dtype, per)
     assert np.sqrt(np.mean(rows ** 2)) <= np.sqrt(np.mean(general ** 2))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("mean,longer", [(6, (20, 40, 49, 80, 200)), (6, (300, 5000)), (20, (49, 60, 100, 1000))])
+def test_longer_rows_among_short_ones(mean, longer, dtype):
+    """Rows of one length with longer ones strewn in: four and more in some groups
+    of 32 rows, none in others, rows that reach over several staged buffers; each
+    length by itself, and the rows around them."""
+    rng = np.random.default_rng(mean + len(longer))
+    lens = np.full(120_000, mean)
+    at = rng.choice(len(lens) // 2, 400 * len(longer), replace=False)     # the second half has none
+    for i, k in enumerate(longer):
+        lens[at[i::len(longer)]] = k
+    assert lens.sum() <= 40 * len(lens)
+    rows, general = _errors(lens, dtype, mean)
+    for k in (mean, *longer):
+        # 400 rows of a length: their root mean square is known to about 4 %
+        slack = 1.0 if k == mean else 1.1
+        sel = lens == k
+        assert np.sqrt(np.mean(rows[sel] ** 2)) <= slack * np.sqrt(np.mean(general[sel] ** 2)), k
