@@ -290,6 +290,7 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.wchains.upload(lay.chains.data(), lay.chains.size(), s);
     F.wcounts.alloc(std::max<size_t>(lay.counts.size(), 16));
     F.wcounts.upload(lay.counts.data(), lay.counts.size(), s);
+    F.row_words = lay.row_words;
     if (chain_major) {
         F.wrows.alloc(std::max<size_t>(lay.rows.size(), 1));
         F.wrows.upload(lay.rows.data(), lay.rows.size(), s);
@@ -306,7 +307,7 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
             L.g0 = lay.colour_groups[c];
             L.g1 = lay.colour_groups[c + 1];
             L.early_x = F.launches.empty() ? 0 : 1;
-            L.smem = ((size_t)lay.colour_slots[c] * 32 * (4 + sizeof(VT)) + 32 * (chain_major ? (bs > 16 ? 8 : 4) : 2) * (size_t)bs + 15) / 16 * 16;
+            L.smem = ((size_t)lay.colour_slots[c] * 32 * (4 + sizeof(VT)) + 32 * (chain_major ? 4 * lay.row_words : 2) * (size_t)bs + 15) / 16 * 16;
             if (L.g1 > L.g0) F.launches.push_back(L);
         }
     } else {
@@ -557,7 +558,7 @@ void launch_cc(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
                                                  L.g0, (const int2 *)F.wchains.p,
                                                  (const unsigned *)F.wrows.p, (const VT *)F.val.p,
                                                  (const int *)F.col.p, (const unsigned char *)F.wicol.p,
-                                                 (const VT *)F.dinv.p, x, y, gate, status, L.early_x));
+                                                 (const VT *)F.dinv.p, x, y, gate, status, L.early_x, F.row_words));
                     continue;
                 }
             }
@@ -565,7 +566,7 @@ void launch_cc(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
                                          (const int2 *)F.wchains.p, (const unsigned *)F.wrows.p,
                                          (const VT *)F.val.p, (const int *)F.col.p,
                                          (const unsigned char *)F.wicol.p, (const VT *)F.dinv.p, x, y, gate, status,
-                                         L.early_x));
+                                         L.early_x, F.row_words));
             continue;
         }
         if constexpr (BS >= 4) {

@@ -68,9 +68,10 @@ size_t wf_bytes_for(int slots, int bs, bool upper)
 
 // What a lane of k_sweep_rl needs of its row: the external entries of the
 // chain's rows solved before it (eo) and its own (ne), the same of in-chain
-// entries (io, left), and the levels of its chain. Chains of up to 16 rows take
-// one word (with distinct columns io <= 120 and left, depth <= 15 there; the
-// builder checks them, as columns may be repeated), longer ones two.
+// entries (io, left), and the levels of its chain. One word where all of a
+// factor's rows fit it, else two: chains of more than 16 rows, rows with 128
+// outside entries or more, columns repeated in a row (distinct ones keep io <= 120
+// and left, depth <= 15 in chains of 16).
 struct RowWord {
     int eo, ne, io, left, depth;
 };
@@ -94,7 +95,8 @@ struct WfLayout {
     std::vector<WfGroup> groups;  // in processing order
     std::vector<int2> chains;     // per group 32 x {first row, E | I << 16} (unused lanes {0, 0})
     std::vector<unsigned char> counts;  // per group 32 x 2*bs row counts (external, in-chain)
-    std::vector<unsigned> rows;   // chain_major: per group 32 x bs row words (row_word; two words a row for bs = 32)
+    std::vector<unsigned> rows;   // chain_major: per group 32 x bs rows of row_words words (row_word)
+    int row_words = 0;
     std::vector<unsigned char> icol;  // chain_major: chain-local columns of the in-chain entries, at their places
     std::vector<VT> val;          // block values
     std::vector<int> col;         // block column words
@@ -110,8 +112,7 @@ struct WfLayout {
 // Builds the layout of one factor. colour_of[row]: the colour's index in
 // processing order. Throws std::invalid_argument when the factor does not fit
 // the schedule; returns false when a group's block would need more than
-// `max_smem` bytes of shared memory per warp, or with chain_major when a row's
-// counts do not fit its word.
+// `max_smem` bytes of shared memory per warp.
 template <typename VT>
 bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const int *cind, const int *rptr,
                     const std::vector<WfColour> &colours, int bs, const int *colour_of, size_t max_smem,
@@ -209,10 +210,9 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
     out.val.assign((size_t)off, VT(0));
     out.col.assign((size_t)off, 0);
     out.counts.assign((size_t)ng * 32 * 2 * bs, 0);
-    const int rw = bs > 16 ? 2 : 1;
-    out.rows.assign(chain_major ? (size_t)ng * 32 * bs * rw : 0, 0u);
+    out.rows.assign(chain_major ? (size_t)ng * 32 * bs * 2 : 0, 0u);
     out.icol.assign(chain_major ? (size_t)off : 0, 0);
-    bool packs = true;
+    bool packs = bs <= 16;  // every row fits one word
     out.cdinv.assign(upper ? (size_t)ng * 32 * bs : 0, VT(0));
     out.dinv.assign(upper ? N : 0, VT(0));
     std::vector<int> owner(N, -1);  // group of each row
@@ -264,21 +264,27 @@ bool make_wf_layout(WfLayout<VT> &out, bool upper, int N, const VT *val, const i
                 for (int st = 0; st < bs; st++) {
                     const int l = upper ? bs - 1 - st : st;
                     const unsigned ne = cnt[l], left = cnt[bs + l];
-                    unsigned *w = &out.rows[(((size_t)g * 32 + q) * bs + l) * rw];
-                    if (rw == 1) {
-                        packs = packs && eo < 1024 && ne < 128 && io < 128 && left < 16;
-                        *w = eo | ne << 10 | io << 17 | left << 24 | depth << 28;
-                    } else {
-                        w[0] = eo | ne << 16 | depth << 24;
-                        w[1] = io | left << 16;
-                    }
+                    unsigned *w = &out.rows[(((size_t)g * 32 + q) * bs + l) * 2];
+                    w[0] = eo | ne << 16 | depth << 24;
+                    w[1] = io | left << 16;
+                    packs = packs && eo < 1024 && ne < 128 && io < 128 && left < 16;
                     eo += ne;
                     io += left;
                 }
             }
         }
     }
-    if (!packs) return false;
+    out.row_words = packs ? 1 : 2;
+    if (chain_major && packs) {
+        std::vector<unsigned> one(out.rows.size() / 2);
+#pragma omp parallel for schedule(static)
+        for (long long i = 0; i < (long long)one.size(); i++) {
+            const RowWord u = row_word(make_uint2(out.rows[2 * i], out.rows[2 * i + 1]));
+            one[i] = (unsigned)u.eo | (unsigned)u.ne << 10 | (unsigned)u.io << 17 | (unsigned)u.left << 24 |
+                     (unsigned)u.depth << 28;
+        }
+        out.rows.swap(one);
+    }
     // dependencies: the groups owning each group's external columns (all earlier)
     std::vector<std::vector<int>> deps(ng);
     bad = -1;

@@ -1,6 +1,7 @@
 """The row-per-lane layout (row words, in-chain columns) on the CPU: its
-emulation against the oracle's sequential sweeps, with columns repeated in a row,
-which a factor may hold, so that a row's counts reach past one word."""
+emulation against the oracle's sequential sweeps, with columns repeated in a row
+(which a factor may hold) and rows of 128 and more outside entries, whose counts
+need two words; and the kernels on the same factors."""
 import ctypes as C
 import os
 import subprocess
@@ -72,6 +73,27 @@ def test_emulated_rows_equal_the_oracle(emu, port, kind, n, bs, times, part, dty
                err, 256)
         assert rc == 0, err.value.decode()
         want = port.sptrsv(F, t, bool(upper)).astype(dtype)
-        if info[0]:                        # 0: the plan takes the row slots
-            assert np.max(np.abs(y - want)) <= tol * np.max(np.abs(want))
+        assert info[0] in (1, 2)           # words a row: the layout takes every factor
+        if bs > 16 or (part is not None and not upper):
+            assert info[0] == 2
+        assert np.max(np.abs(y - want)) <= tol * np.max(np.abs(want))
         t = want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sweep", [L.SWEEP_ROWS, L.SWEEP_ROWS_WIDE])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind,n,bs,times,part", [c for c in CASES if c[4]])
+def test_sweeps_of_two_words_a_row(port, kind, n, bs, times, part, dtype, sweep):
+    import torch
+    from test_gpu_kernels import Plan
+    Lf, Uf, nc, sc = factors(kind, n, bs, times, part, dtype)
+    pl = Plan(Lf, Uf, L.PC_ILU_ABMC, sc, nc, bs, dtype, sweep=sweep)
+    L.check("plan", pl.code)
+    x = np.random.default_rng(6).uniform(-1, 1, Lf.n).astype(dtype)
+    y = torch.from_numpy(x).cuda()
+    L.check("apply", L.lib().senk_ilu_plan_apply(pl.h, y.data_ptr(), y.data_ptr(), None))
+    L.check("status", L.lib().senk_ilu_plan_status(pl.h, None))
+    want = port.sptrsv(Uf, port.sptrsv(Lf, x, False), True)
+    tol = 1e-12 if dtype == np.float64 else 1e-5
+    assert np.max(np.abs(y.cpu().numpy() - want)) <= tol * np.max(np.abs(want))
