@@ -147,7 +147,6 @@ struct BlGroup {
 
 constexpr int kBlMaxSteps = 16;
 constexpr size_t kBlMaxSmem = 160 * 1024;  // shared memory of a group; the kernels' limit for every plan
-constexpr int kBlMaxGroups = 14;  // to an SM, mean of the colours, FP64 (IlubPlan::build_slices)
 
 // Byte offsets of a group's staged part: widths (external, in-chain) of each
 // step, the external block columns, the in-chain columns (scalar, from the
@@ -580,13 +579,11 @@ bool IlubPlan<T>::build_slices(bool upper, const int *bcind, const int *brptr, c
         if ((int)gd.size() > before) F.launches.push_back({before, (int)gd.size(), 0});
     }
     const int ng = (int)gd.size();
-    // FP64 colours of many groups to an SM: k_ilub_sweep, which then has enough
-    // chains to hide its latencies, reads y and the factor once and no padding.
-    // Block-3x3 system: 10.5 groups to an SM and colour (80^3 nodes) 0.430 ms
-    // against its 0.623, GCR(20) 17.4 against 20.9; 18.2 (96^3) 0.720 against
-    // 0.752, but GCR(20), its vectors and factors cold, 34.6 against 31.2 (with four
-    // slots ahead, 0.778). FP32 is faster in slices there too (0.317 against 0.472).
-    if (sizeof(T) == 8 && ng > (long long)kBlMaxGroups * sm_count() * (long long)F.launches.size()) return false;
+    // at any width: 3x3 blocks, 10.5 to 28.9 groups to an SM and colour (80^3 to 112^3
+    // nodes), one FP64 application and 20 GCR iterations against k_ilub_sweep's:
+    // 0.43 : 0.62 ms and 17.3 : 20.5 at 10.5, 0.57 : 0.73 and 22.6 : 25.5 at 14, 0.72 :
+    // 0.75 and 28.7 : 28.6 at 18.2, 0.77 : 1.07 and 31.4 : 37.0 at 20.6, 1.03 : 1.45 and
+    // 42.9 : 51.2 at 28.9
     std::vector<uint16_t> widths((size_t)ng * 2 * per, 0);
     bool fits = true;
 #pragma omp parallel for schedule(static) reduction(&& : fits)
