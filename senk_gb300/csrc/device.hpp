@@ -45,6 +45,13 @@ int guarded(const char *fn, F &&body)
     }
 }
 
+// Bytes that this thread has uploaded through DevBuf.
+inline long long &uploaded_bytes()
+{
+    static thread_local long long n = 0;
+    return n;
+}
+
 // Owning device allocation.
 template <typename T>
 struct DevBuf {
@@ -76,6 +83,7 @@ struct DevBuf {
     void upload(const T *h, size_t count, cudaStream_t s)
     {
         if (count) SENK_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
+        uploaded_bytes() += (long long)(count * sizeof(T));
     }
     void upload(const std::vector<T> &h, cudaStream_t s)
     {
@@ -313,11 +321,6 @@ struct IlubPlan {
         sweep(true, (const T *)y, y, s, gate);
     }
     long long apply_bytes() const;
-    long long h2d_bytes() const
-    {
-        const long long bs = (long long)bnl * bnw;
-        return (lblocks + ublocks) * (bs * (long long)sizeof(T) + 4) + 2LL * (nbr + 1) * 4 + (long long)chains.bytes();
-    }
 };
 
 // --------------------------------------------------------- Krylov system

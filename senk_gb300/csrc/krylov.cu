@@ -90,6 +90,7 @@ void System<T>::create(const senk_system_desc &d, const senk_options *o, cudaStr
         A.upload((const T *)d.val, d.cind, d.rptr, n, opt.spmv, stream, !(sell_only || ir_only) || d.mixed);
     }
     clk.lap("A upload (+SELL build)");
+    const long long before = uploaded_bytes();
     if (ir_only) {
         // nothing to build here for the preconditioner
     } else if (d.precond == SENK_PC_ILUB || d.precond == SENK_PC_ILUB_ABMC) {
@@ -103,6 +104,7 @@ void System<T>::create(const senk_system_desc &d, const senk_options *o, cudaStr
         pc->build(n, (const T *)d.lval, d.lcind, d.lrptr, (const T *)d.uval, d.ucind, d.urptr, d.precond, d.cptr,
                   d.cnum, d.bsize, stream, opt.sweep);
     }
+    h2d_bytes = A.h2d + uploaded_bytes() - before;  // A, and what the plan was built from
     clk.lap("preconditioner plan");
     b.alloc(n);
     x.alloc(n);
@@ -114,13 +116,6 @@ void System<T>::create(const senk_system_desc &d, const senk_options *o, cudaStr
     if (d.m_max > 0 && !ir_only) ensure_gmres(d.m_max);
     SENK_CUDA(cudaStreamSynchronize(stream));
     clk.lap("vectors + Krylov workspace");
-    h2d_bytes = A.h2d;
-    if (pcb) h2d_bytes += pcb->h2d_bytes();
-    if (pc) {
-        for (const SweepFactor<T> *F : {&pc->L, &pc->U})
-            h2d_bytes += (long long)(F->val.bytes() + F->col.bytes() + F->dinv.bytes() + F->rowmap.bytes() +
-                                     F->groups.bytes() + F->widths.bytes() + F->lblocks.bytes() + F->blocks.bytes());
-    }
     if (d.mixed) {
         SENK_REQUIRE(sizeof(T) == sizeof(double), "mixed precision needs an FP64 system");
         // FP32 copies of A and the factors, as senk::utils::Convert makes them
