@@ -183,7 +183,7 @@ struct SweepFactor {
     bool compact = false;          // compact chain layout (else row slots)
     bool dataflow = false;         // compact: one launch per sweep (else one per colour)
     std::vector<int> colour_slots; // compact: widest block of each colour
-    DevBuf<unsigned char> wcounts; // compact: per chain, external and in-chain counts of each row
+    DevBuf<unsigned char> wcounts; // compact, not rowlane: per chain, external and in-chain counts of each row
     DevBuf<unsigned> wrows;        // compact, rowlane: row words (row_word), row_words to a row
     int row_words = 1;
     DevBuf<unsigned char> wicol;   // compact, rowlane: chain-local columns of the in-chain entries

@@ -288,10 +288,11 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     F.wgroups.upload(lay.groups.data(), ng, s);
     F.wchains.alloc(std::max<size_t>(lay.chains.size(), 1));
     F.wchains.upload(lay.chains.data(), lay.chains.size(), s);
-    F.wcounts.alloc(std::max<size_t>(lay.counts.size(), 16));
-    F.wcounts.upload(lay.counts.data(), lay.counts.size(), s);
     F.row_words = lay.row_words;
-    if (chain_major) {
+    if (!chain_major) {
+        F.wcounts.alloc(std::max<size_t>(lay.counts.size(), 16));
+        F.wcounts.upload(lay.counts.data(), lay.counts.size(), s);
+    } else {
         F.wrows.alloc(std::max<size_t>(lay.rows.size(), 1));
         F.wrows.upload(lay.rows.data(), lay.rows.size(), s);
         F.wicol.alloc(std::max<size_t>(lay.icol.size(), 16));
@@ -324,6 +325,10 @@ bool build_factor_wf(SweepFactor<VT> &F, bool upper, int N, const VT *val, const
     SENK_CUDA(cudaStreamSynchronize(s));  // the layout's host arrays are released on return
     return true;
 }
+
+// Which factors take the row-sorted slices (the others' rules: IluPlan::build).
+template <typename VT>
+constexpr bool kSlices = sizeof(VT) == 8;
 
 // Most bytes of entries a group should have, so that four CTAs of k_sweep_lv
 // are resident per SM with its operands.
@@ -777,11 +782,13 @@ template <typename VT, typename XT, bool UPPER>
 void sweep_groups(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaStream_t s, const int *gate)
 {
     const int nc = (int)F.colour_groups.size() - 1;
-    if (F.slices) {
-        static_assert(std::is_same<VT, XT>::value, "factor and vector types agree");
-        launch_lv<VT, UPPER>(F, status, x, y, s, gate);
-        SENK_LAUNCH_CHECK();
-        return;
+    if constexpr (kSlices<VT>) {
+        if (F.slices) {
+            static_assert(std::is_same<VT, XT>::value, "factor and vector types agree");
+            launch_lv<VT, UPPER>(F, status, x, y, s, gate);
+            SENK_LAUNCH_CHECK();
+            return;
+        }
     }
     if (F.compact) {
 #define SENK_COMPACT_CASE(BS)                                                      \
@@ -996,7 +1003,7 @@ void IluPlan<VT>::build(int N, const VT *lval, const int *lcind, const int *lrpt
     // one launch per sweep. A factor whose groups do not fit shared memory
     // falls back to row slots.
     const bool persistent = sweep_mode == SENK_SWEEP_PERSISTENT;
-    const bool slices = sweep_mode == SENK_SWEEP_AUTO && sizeof(VT) == 8;
+    const bool slices = sweep_mode == SENK_SWEEP_AUTO && kSlices<VT>;
     const bool rows = sweep_mode == SENK_SWEEP_ROWS || sweep_mode == SENK_SWEEP_ROWS_WIDE ||
                       (sweep_mode == SENK_SWEEP_AUTO && !slices);
     const bool wide = sweep_mode == SENK_SWEEP_WIDE || sweep_mode == SENK_SWEEP_ROWS_WIDE;
@@ -1006,9 +1013,13 @@ void IluPlan<VT>::build(int N, const VT *lval, const int *lcind, const int *lrpt
     auto build_one = [&](SweepFactor<VT> &F, auto upper, const VT *v, const int *c, const int *r,
                          const std::vector<Group> &colours) {
         constexpr bool kUpper = decltype(upper)::value;
-        if (slices && build_factor_lv<VT, kUpper>(F, N, v, c, r, colours, bs, colour_of, s)) {
-            shape_lv<VT, kUpper>(F);
-        } else if (compact && build_factor_wf(F, kUpper, N, v, c, r, colours, bs, colour_of, df, s, nullptr, rows)) {
+        if constexpr (kSlices<VT>) {
+            if (slices && build_factor_lv<VT, kUpper>(F, N, v, c, r, colours, bs, colour_of, s)) {
+                shape_lv<VT, kUpper>(F);
+                return;
+            }
+        }
+        if (compact && build_factor_wf(F, kUpper, N, v, c, r, colours, bs, colour_of, df, s, nullptr, rows)) {
             F.persistent = persistent;
             F.force_wide = wide;
             shape_wf_bs<VT, kUpper>(F);
