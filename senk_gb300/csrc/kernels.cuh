@@ -2134,12 +2134,12 @@ constexpr int rl_min_blocks(int bs, int r, int vbytes)
 // offsets by one shuffle scan of the chain's counts. Prologue, programmatic
 // launch, early_x and gate as in k_sweep_cc; a staging wait that runs out sets
 // *status = 2 and its warp leaves (after a second bounded wait for the copy).
-template <typename VT, typename XT, int BS, bool UPPER, int R>
+template <typename VT, typename XT, int BS, bool UPPER, int R, bool TWO>
 __global__ void __launch_bounds__(BS * 32 / R,
                                   rl_min_blocks(BS, R, (int)(sizeof(VT) > sizeof(XT) ? sizeof(VT) : sizeof(XT))))
 k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ chains,
            const unsigned *__restrict__ rows, const VT *__restrict__ val, const int *__restrict__ col,
-           const unsigned char *__restrict__ icol, const VT *__restrict__ dinv, const XT *x, XT *y, const int *gate, int *status, int early_x, int words)
+           const unsigned char *__restrict__ icol, const VT *__restrict__ dinv, const XT *x, XT *y, const int *gate, int *status, int early_x)
 {
     static_assert(R == 1 || (R == 2 && BS >= 2), "two chains per lane need chains of at least two rows");
     constexpr int CPW = 32 / BS;  // chains per warp, per r
@@ -2152,12 +2152,12 @@ k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
     // external columns, values of all entries, in-chain columns (a byte each), row words
     const unsigned cbytes = (unsigned)d.emax * 32u * 4u, ibytes = (unsigned)d.imax * 32u,
                    vbytes = (unsigned)slots * 32u * (unsigned)sizeof(VT);
-    const bool two = BS > 16 || words == 2;  // words of a row
-    const unsigned nbytes = 32u * BS * (two ? 8u : 4u);
+    using RW = typename std::conditional<TWO, uint2, unsigned>::type;  // the words of a row
+    constexpr unsigned nbytes = 32u * (unsigned)sizeof(RW) * BS;
     const int *cw = reinterpret_cast<const int *>(ccs);
     const VT *vw = reinterpret_cast<const VT *>(ccs + cbytes);
     const unsigned char *ic = ccs + cbytes + vbytes;
-    const unsigned *info = reinterpret_cast<const unsigned *>(ic + ibytes);
+    const RW *info = reinterpret_cast<const RW *>(ic + ibytes);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         mbar_expect_tx(&bar, cbytes + vbytes + ibytes + nbytes);
@@ -2216,8 +2216,7 @@ k_sweep_rl(const WfGroup *__restrict__ groups, int g0, const int2 *__restrict__ 
     int ea[R], ne[R], ia[R], left[R], nmax = 0, depth = 0, longest = 0;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        const int at = qc[r] * BS + rr;
-        const RowWord u = two ? row_word(reinterpret_cast<const uint2 *>(info)[at]) : row_word(info[at]);
+        const RowWord u = row_word(info[qc[r] * BS + rr]);
         ea[r] = qc[r] * d.emax + u.eo;
         ne[r] = u.ne;
         ia[r] = ib[r] + u.io;

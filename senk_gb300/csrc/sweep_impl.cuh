@@ -521,6 +521,22 @@ void launch_wf(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
                                  F.flags.p, F.ctrl.p, x, y, gate, status, F.slots_max));
 }
 
+// The form of k_sweep_rl for rows of `words` words (chains of more than 16 rows:
+// always two), with two chains a lane if `wide`.
+template <typename VT, typename XT, int BS, bool UPPER>
+auto row_kernel(int words, bool wide) -> decltype(&k_sweep_rl<VT, XT, BS, UPPER, 1, true>)
+{
+    if constexpr (BS >= 2)
+        if (wide) {
+            if constexpr (BS <= 16)
+                if (words == 1) return k_sweep_rl<VT, XT, BS, UPPER, 2, false>;
+            return k_sweep_rl<VT, XT, BS, UPPER, 2, true>;
+        }
+    if constexpr (BS <= 16)
+        if (words == 1) return k_sweep_rl<VT, XT, BS, UPPER, 1, false>;
+    return k_sweep_rl<VT, XT, BS, UPPER, 1, true>;
+}
+
 // Compact chains, one launch per colour (k_sweep_cc), chained by programmatic
 // dependent launch.
 template <typename VT, typename XT, int BS, bool UPPER>
@@ -556,22 +572,12 @@ void launch_cc(const SweepFactor<VT> &F, int *status, const XT *x, XT *y, cudaSt
         cfg.attrs = at;
         cfg.numAttrs = 1;
         if (F.rowlane) {
-            if constexpr (BS >= 2) {
-                if (L.wide) {
-                    cfg.blockDim = dim3(BS * 16);
-                    SENK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep_rl<VT, XT, BS, UPPER, 2>, (const WfGroup *)F.wgroups.p,
-                                                 L.g0, (const int2 *)F.wchains.p,
-                                                 (const unsigned *)F.wrows.p, (const VT *)F.val.p,
-                                                 (const int *)F.col.p, (const unsigned char *)F.wicol.p,
-                                                 (const VT *)F.dinv.p, x, y, gate, status, L.early_x, F.row_words));
-                    continue;
-                }
-            }
-            SENK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep_rl<VT, XT, BS, UPPER, 1>, (const WfGroup *)F.wgroups.p, L.g0,
-                                         (const int2 *)F.wchains.p, (const unsigned *)F.wrows.p,
-                                         (const VT *)F.val.p, (const int *)F.col.p,
+            auto kern = row_kernel<VT, XT, BS, UPPER>(F.row_words, L.wide);
+            if (L.wide) cfg.blockDim = dim3(BS * 16);
+            SENK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const WfGroup *)F.wgroups.p, L.g0, (const int2 *)F.wchains.p,
+                                         (const unsigned *)F.wrows.p, (const VT *)F.val.p, (const int *)F.col.p,
                                          (const unsigned char *)F.wicol.p, (const VT *)F.dinv.p, x, y, gate, status,
-                                         L.early_x, F.row_words));
+                                         L.early_x));
             continue;
         }
         if constexpr (BS >= 4) {
@@ -599,9 +605,11 @@ template <typename VT, int BS, bool UPPER>
 void shape_cc(SweepFactor<VT> &F)
 {
     if (F.rowlane) {
-        allow_dynamic(k_sweep_rl<VT, VT, BS, UPPER, 1>, kMaxWfSmem);
+        auto one_kern = row_kernel<VT, VT, BS, UPPER>(F.row_words, false);
+        allow_dynamic(one_kern, kMaxWfSmem);
         if constexpr (BS >= 2) {
-            allow_dynamic(k_sweep_rl<VT, VT, BS, UPPER, 2>, kMaxWfSmem);
+            auto two_kern = row_kernel<VT, VT, BS, UPPER>(F.row_words, true);
+            allow_dynamic(two_kern, kMaxWfSmem);
             for (auto &L : F.launches) {
                 if (L.coop) continue;
                 if (F.force_wide) {
@@ -609,10 +617,8 @@ void shape_cc(SweepFactor<VT> &F)
                     continue;
                 }
                 int one = 0, two = 0;
-                SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_sweep_rl<VT, VT, BS, UPPER, 1>,
-                                                                        BS * 32, L.smem));
-                SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, k_sweep_rl<VT, VT, BS, UPPER, 2>,
-                                                                        BS * 16, L.smem));
+                SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, one_kern, BS * 32, L.smem));
+                SENK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, two_kern, BS * 16, L.smem));
                 L.wide = (L.g1 - L.g0) > one * sm_count() && two > one ? 1 : 0;
             }
         }
