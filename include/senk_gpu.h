@@ -61,7 +61,8 @@ typedef struct {
 #define SENK_ORTH_MGS 2  /* modified Gram-Schmidt, the reference's order */
 
 #define SENK_SPMV_AUTO 0  /* SELL-32-sigma(256) for the solver's SpMV */
-#define SENK_SPMV_CSR 1   /* CSR, lanes per row from the mean row length */
+#define SENK_SPMV_CSR 1   /* CSR: a lane per row up to a mean of 40 entries, else
+                             several by the mean row length */
 #define SENK_SPMV_SELL 2  /* SELL-32 built on upload, rows in order */
 #define SENK_SPMV_SELL_SIGMA 3 /* SELL-32-sigma: within each window of 256 rows
                                   the rows are taken longest first (stable) before

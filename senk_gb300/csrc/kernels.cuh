@@ -2127,13 +2127,14 @@ constexpr int rl_min_blocks(int bs, int r, int vbytes)
 // applications, their bytes: hence a byte per in-chain column and a word per
 // row. FP32 application 128^3 83.4 -> 78.2 us, 160^3 132.9 -> 126.8, 76^3 49.5
 // -> 45.9, 48^3 44.3 -> 40.6 (before: ChainRec, counts scanned by shuffles).
-// Each lane stores its row; after the staging wait no CTA barrier is needed. R = 2 (BS >= 2) halves the
-// threads of a group, for colours with more groups than one wave of R = 1
-// holds. Each lane reads its chains' descriptors itself (the chain-major
-// layout stores the chain's in-chain offset there) and finds its row's
-// offsets by one shuffle scan of the chain's counts. Prologue, programmatic
-// launch, early_x and gate as in k_sweep_cc; a staging wait that runs out sets
-// *status = 2 and its warp leaves (after a second bounded wait for the copy).
+// Each lane stores its row; after the staging wait no CTA barrier is needed. R = 2
+// (BS >= 2) halves the threads of a group, for colours with more groups than one
+// wave of R = 1 holds. Each lane reads its chains' descriptors itself (the
+// chain-major layout stores the chain's in-chain offset there); its row's offsets
+// and counts are the row's word, or two with TWO (row_word). Prologue,
+// programmatic launch, early_x and gate as in k_sweep_cc; a staging wait that runs
+// out sets *status = 2 and its warp leaves (after a second bounded wait for the
+// copy).
 template <typename VT, typename XT, int BS, bool UPPER, int R, bool TWO>
 __global__ void __launch_bounds__(BS * 32 / R,
                                   rl_min_blocks(BS, R, (int)(sizeof(VT) > sizeof(XT) ? sizeof(VT) : sizeof(XT))))

@@ -1,5 +1,5 @@
 // Builds the row-sorted slice layout (lv_layout.hpp) on the device from the
-// factor's CSR arrays; the blocks equal make_lv_layout's byte for byte. On the
+// factor's CSR arrays, in the form and order of make_lv_layout's blocks. On the
 // host the layout costs several times what the row slots did (sorting and
 // finding the distinct columns of every group); here one CTA builds a group,
 // once for its size and once more to write it.

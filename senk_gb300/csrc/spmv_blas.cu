@@ -19,9 +19,10 @@ int csr_lanes(long long nnz, int n)
 
 namespace {
 
-// Longest mean row that k_spmv_csr_rows takes. Measured at 27 entries per row:
-// FP64 89 us against 345 us for the lanes, FP32 49 against 95; at 81: FP64 96
-// against 101, FP32 51 against 33 (few warps' buffers fit an SM then).
+// Longest mean row that k_spmv_csr_rows takes. Measured on 884,736 rows, L2 flushed:
+// 27 entries FP64 101 us against 373 us for the lanes, FP32 60 against 132; 40: 160
+// against 472 and 97 against 165; 48: 271 against 472, but 166 against 162 (few
+// warps' buffers fit an SM then).
 constexpr int kRowsMean = 40;
 
 // Shared memory that an SM's warps of k_spmv_csr_rows may take; a CTA takes a
